@@ -10,8 +10,23 @@
 // Structure of one CTA (192 threads, one CTA per SM, static round-robin tile schedule):
 //   warp 0      TMA producer: cp.async.bulk.tensor tiles into a 128B-swizzled smem ring
 //   warp 1      allocates TMEM; one lane issues tcgen05.mma and tcgen05.commit
-//   warps 2..5  epilogue: tcgen05.ld the finished accumulator, convert, store to global
+//   warps 2..5  epilogue: tcgen05.ld the finished accumulator, convert, stage in smem, TMA store / reduce
 // Two TMEM accumulators let the epilogue of tile i overlap the main loop of tile i+1.
+//
+// CG = 2: a cluster of two CTAs works on one 256 x BN tile (`cta_group::2`). Each CTA holds its 128 rows of A and HALF
+// of B's BN rows in its shared memory and accumulates its own 128 x BN half; the even CTA issues the products for both.
+// Per 64-deep k-block an SM then fetches 16 KB + BN * 64 B instead of 16 KB + BN * 128 B, so the L2 and the
+// shared-memory port carry a third less at BN = 256, and a tile of the pair needs half as many loads of A.
+//
+// The output leaves through shared memory and TMA (whole 128-byte row segments) instead of one 16-byte store per lane
+// and row: the scattered stores, not the tensor pipe, bounded the short contractions (4096 x 7168 x 1280: 67 us with
+// them; the same main loop with the cross-entropy epilogue, which stores nothing, ran at 1.6 PFLOP/s). fp32 C += is a
+// TMA reduction for the same reason. Before / after (one CTA with per-lane stores, stream-K for C +=), B200, us:
+//   4096 x 7168 x 1280  67.4 / 54.6    16384 x 1536 x 4096  246 / 145    16384 x 1536 x 8192 (B MN)  420 / 286
+//   C +=, both MN: 7168 x 1280 x 4096  74.6 / 56.2    8192 x 1536 x 16384  468 / 301    65536 x 1280 x 4096  647 / 490
+// What bounds it now: 8192^3 runs at 1.53 PFLOP/s with 12 TB/s of operands from the L2 (the pair's 256 x 256 tile is
+// the largest that TMEM can double-buffer); products of one to three rounds lose their last, partly empty round and
+// about 4 us of launch, fill and drain.
 // Takes the role of the cuBLAS calls behind nn.Linear in the reference
 // (src/kohakuwullm/models/components/attention.py:77-89, mlp.py:15-126).
 #include "common.cuh"
@@ -22,41 +37,49 @@
 
 namespace kwu {
 
-constexpr int GEMM_BM = 128;
+constexpr int GEMM_BM = 128;  // rows of one CTA
 constexpr int GEMM_BK = 64;   // 64 bf16 = one 128-byte swizzle row
 constexpr int GEMM_THREADS = 192;
+
+// How the accumulator leaves the kernel (EPI_STORE)
+constexpr int OUT_TMA_BF16 = 0;   // bf16, TMA store
+constexpr int OUT_TMA_F32 = 1;    // fp32, TMA store
+constexpr int OUT_TMA_ADD = 2;    // fp32, TMA reduction (C +=)
+constexpr int OUT_DIRECT = 3;     // per-lane stores: scattered rows, bf16 C +=, pitches TMA cannot address
 
 struct GemmParams {
   int M, N, K;
   int ldc;
+  int bn;           // width of a tile
   int out_fp32;     // 0: bf16 output, 1: fp32 output
-  int accumulate;   // 1: C += A*B (read-modify-write in the epilogue)
+  int accumulate;   // 1: C += A*B
+  int out_mode;     // OUT_*
+  int out_cols;     // bf16 TMA stores: columns of one store box (64, or 32 when bn is not a multiple of 64)
   float alpha;      // scale applied to the product
   // descriptor constants, computed on the host
   uint32_t a_lbo, a_sbo, a_kadv;
   uint32_t b_lbo, b_sbo, b_kadv;
   uint32_t idesc;
-  int tiles_m, tiles_n;
+  uint32_t stage_bytes;   // one ring stage of one CTA: its A rows and its share of B
+  int b_chunks;           // MN-major B: 64-column boxes of one CTA's share
+  int stages;
+  int tiles_m, tiles_n;   // tile grid (a tile is 128 * CG rows)
   int* status;
-  // split-K (group_mode 0 only): the contraction is cut into `splits` ranges handled by different CTAs,
-  // each adding its partial product into the fp32 output with vector reductions (needs out_fp32 and
-  // C += semantics). Used by weight gradients, whose outputs have too few tiles to fill the GPU.
-  int splits;
-  // stream-K (group_mode 0 only, fp32 C += semantics): the (tile, k-block) work units are cut into
-  // `streamk` equal contiguous ranges, one per CTA; a CTA adds the partial product of every tile its range
-  // touches into the output with vector reductions, so all SMs finish together whatever the tile count.
-  int streamk;
+  // split tail (fp32 C += only): tiles [0, full_tiles) are whole work items; each of the `tail_tiles` after them, which
+  // would leave the last round of the persistent grid partly empty, is cut into `splits` ranges of the contraction for
+  // CTAs (pairs) that would idle, all adding into C. 0 tail tiles: every tile is a whole item.
+  int full_tiles, tail_tiles, splits;
   // grouped (mixture-of-experts) modes
   //   1: rows grouped by expert: row tile t reads group_tiles[t] = (m0, expert, valid); the expert picks
   //      a block of `group_b_rows` rows of B (K-major: output rows; MN-major: contraction rows)
   //   2: contraction grouped by expert (weight gradients): C[e] (+)= A[rows_e]^T B[rows_e] with
-  //      rows_e = [group_offsets[e], group_offsets[e+1]); C advances by c_group_stride elements per expert
+  //      rows_e = [group_offsets[e], group_offsets[e+1]); C advances by c_group_rows rows per expert
   int group_mode;
   const int4* group_tiles;
   const int* group_offsets;
   int group_b_rows;
   int num_groups;
-  long long c_group_stride;
+  int c_group_rows;
   // scatter epilogue (bf16 EPI_STORE only): output row r goes to the byte address row_ptrs[r] (0: row is
   // dropped) instead of C + r*ldc. The addresses may be peer-mapped memory of another GPU: the expert-
   // parallel combine / gradient return is then done by the GEMM's own epilogue stores, tile by tile.
@@ -74,135 +97,128 @@ constexpr int EPI_STORE = 0;    // C (+)= alpha * acc
 constexpr int EPI_LSE = 1;      // no C: per-row (max, sum-exp) partials and the target logit
 constexpr int EPI_DLOGITS = 2;  // C = coef_p * exp(acc - lse) - coef_y * onehot   (bf16)
 
-template <int BN>
-struct GemmSmem {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
-  static constexpr int B_BYTES = BN * GEMM_BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN >= 256) ? 4 : ((BN >= 192) ? 5 : 6);
-  static constexpr int BAR_BYTES = 1024;
-  // per epilogue warp a 32 x 32 fp32 patch (rows padded to 36 floats) through which the fp32 reductions are
-  // transposed, so that one warp instruction adds to 4 rows x 128 contiguous bytes instead of 32 rows x 16 bytes
-  static constexpr int RED_STAGE_BYTES = 4 * 32 * 36 * 4;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + BAR_BYTES + RED_STAGE_BYTES + 1024;  // +1024 alignment slack
-};
+constexpr int GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;
+constexpr int GEMM_MAX_STAGES = 8;
+constexpr int GEMM_BAR_BYTES = 1024;
+// per epilogue warp two 4 KB patches (32 rows x 128 bytes) that TMA stores read
+constexpr int GEMM_OUT_BYTES = 4 * 2 * 4096;
+constexpr int GEMM_SMEM_MAX = 227 * 1024;
 
 struct TileInfo {
   int m0, n0;        // output tile origin
   int b_row_off;     // added to B's row coordinate (expert selection)
   int k_begin, nkb;  // contraction range in elements / 64-blocks
-  long long c_off;   // added to the output pointer (elements)
+  int c_row_off;     // added to the output row (expert selection)
 };
 
-constexpr int GEMM_RASTER_M = 16;
+constexpr int GEMM_RASTER_ROWS = 2048;
 
 // Same decoding in every role of the CTA. Returns false for tiles that carry no work.
-template <int BN>
+template <int CG>
 __device__ __forceinline__ bool decode_tile(const GemmParams& p, int tile, int num_kb, TileInfo& t) {
-  t.b_row_off = 0; t.k_begin = 0; t.nkb = num_kb; t.c_off = 0;
+  constexpr int TM = GEMM_BM * CG;
+  t.b_row_off = 0; t.k_begin = 0; t.nkb = num_kb; t.c_row_off = 0;
   if (p.group_mode == 2) {
     const int per = p.tiles_m * p.tiles_n;
     const int e = tile / per, r = tile % per;
-    t.m0 = (r / p.tiles_n) * GEMM_BM;
-    t.n0 = (r % p.tiles_n) * BN;
+    t.m0 = (r / p.tiles_n) * TM;
+    t.n0 = (r % p.tiles_n) * p.bn;
     t.k_begin = p.group_offsets[e];
     t.nkb = (p.group_offsets[e + 1] - t.k_begin) / GEMM_BK;
-    t.c_off = static_cast<long long>(e) * p.c_group_stride;
+    t.c_row_off = e * p.c_group_rows;
     return t.nkb > 0;
-  }
-  if (p.splits > 1) {
-    const int per = p.tiles_m * p.tiles_n;
-    const int sidx = tile / per;
-    tile = tile % per;
-    const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * sidx / p.splits);
-    const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (sidx + 1) / p.splits);
-    t.k_begin = kb0 * GEMM_BK;
-    t.nkb = kb1 - kb0;
   }
   if (p.group_mode == 1) {
     const int tm = tile / p.tiles_n;
-    t.n0 = (tile % p.tiles_n) * BN;
+    t.n0 = (tile % p.tiles_n) * p.bn;
     const int4 g = p.group_tiles[tm];
     t.m0 = g.x;
     t.b_row_off = g.y * p.group_b_rows;
     return g.z != 0;
   }
-  // Raster order: panels of GEMM_RASTER_M row tiles, rows fastest inside a panel. The tiles that run at the
+  // Raster order: panels of GEMM_RASTER_ROWS rows, rows fastest inside a panel. The tiles that run at the
   // same time then share a few B tiles and one A panel, which stays in L2; with columns fastest every wave
   // of a wide product (a 65536-row vocabulary matrix) streams a different stretch of B from HBM for every
   // row tile, 32 times the matrix in total.
-  const int span = GEMM_RASTER_M * p.tiles_n;
+  constexpr int RASTER = GEMM_RASTER_ROWS / TM;
+  const int span = RASTER * p.tiles_n;
   const int panel = tile / span, within = tile - panel * span;
-  const int gm = min(GEMM_RASTER_M, p.tiles_m - panel * GEMM_RASTER_M);
-  t.m0 = (panel * GEMM_RASTER_M + within % gm) * GEMM_BM;
-  t.n0 = (within / gm) * BN;
+  const int gm = min(RASTER, p.tiles_m - panel * RASTER);
+  t.m0 = (panel * RASTER + within % gm) * TM;
+  t.n0 = (within / gm) * p.bn;
   return true;
 }
 
-// Work item number `i` of this CTA. 0: none left; 1: `t` holds work; 2: nothing to do for this index, go on.
-template <int BN>
+// Work item number `i` of this CTA (pair). 0: none left; 1: `t` holds work; 2: nothing to do for this index, go on.
+template <int CG>
 __device__ __forceinline__ int next_work(const GemmParams& p, int i, int num_tiles, int num_kb, TileInfo& t) {
-  if (p.streamk > 0) {
-    const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * num_kb;
-    const long long u0 = units * blockIdx.x / p.streamk, u1 = units * (blockIdx.x + 1) / p.streamk;
-    const long long tile = u0 / num_kb + i;
-    const long long start = max(u0, tile * num_kb), end = min(u1, (tile + 1) * num_kb);
-    if (start >= end) return 0;
-    t.b_row_off = 0; t.c_off = 0;
-    t.m0 = static_cast<int>(tile / p.tiles_n) * GEMM_BM;
-    t.n0 = static_cast<int>(tile % p.tiles_n) * BN;
-    t.k_begin = static_cast<int>(start - tile * num_kb) * GEMM_BK;
-    t.nkb = static_cast<int>(end - start);
+  const int item = static_cast<int>(blockIdx.x) / CG + i * (static_cast<int>(gridDim.x) / CG);
+  if (p.tail_tiles > 0 && item >= p.full_tiles) {
+    const int piece = item - p.full_tiles;
+    if (piece >= p.tail_tiles * p.splits) return 0;
+    decode_tile<CG>(p, p.full_tiles + piece % p.tail_tiles, num_kb, t);
+    const int s = piece / p.tail_tiles;
+    const int kb0 = num_kb * s / p.splits, kb1 = num_kb * (s + 1) / p.splits;
+    t.k_begin = kb0 * GEMM_BK;
+    t.nkb = kb1 - kb0;
     return 1;
   }
-  const int tile = blockIdx.x + i * gridDim.x;
-  if (tile >= num_tiles) return 0;
-  return decode_tile<BN>(p, tile, num_kb, t) ? 1 : 2;
+  if (item >= num_tiles) return 0;
+  return decode_tile<CG>(p, item, num_kb, t) ? 1 : 2;
 }
 
-template <int BN, bool A_MN, bool B_MN, int EPI>
+template <int CG, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 void* __restrict__ Cbase, const GemmParams p) {
-  using S = GemmSmem<BN>;
-  constexpr int STAGES = S::STAGES;
-  constexpr uint32_t TMEM_COLS = (2 * BN <= 256) ? 256 : 512;
+                 const __grid_constant__ CUtensorMap tmC, void* __restrict__ Cbase, const GemmParams p) {
+  constexpr uint32_t TMEM_COLS = 512;
 
   extern __shared__ uint8_t smem_raw[];
+  // both CTAs of a pair see the same offset: dynamic shared memory starts at one address in every CTA
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* bar_area = smem + STAGES * S::STAGE_BYTES;
+  uint8_t* out_area = smem;
+  uint8_t* ring = smem + GEMM_OUT_BYTES;
+  uint8_t* bar_area = ring + p.stages * p.stage_bytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(bar_area);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* acc_full = empty_bar + STAGES;
+  uint64_t* empty_bar = full_bar + GEMM_MAX_STAGES;
+  uint64_t* acc_full = empty_bar + GEMM_MAX_STAGES;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* red_stage = reinterpret_cast<float*>(bar_area + S::BAR_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_tiles = p.tiles_m * p.tiles_n * (p.group_mode == 2 ? p.num_groups : 1) * (p.splits > 1 ? p.splits : 1);
+  const int cta = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int num_tiles = p.tiles_m * p.tiles_n * (p.group_mode == 2 ? p.num_groups : 1);
   const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
+  const int BN = p.bn;
+  const int stages = p.stages;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], 128);
+      mbar_init(&acc_empty[s], 4 * CG);   // one arrival per epilogue warp of the pair
     }
     *abort_flag = 0;
     mbar_fence_init();
   }
+  if (warp == 0 && elect_one()) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    if (EPI != EPI_LSE && p.out_mode != OUT_DIRECT) tma_prefetch_desc(&tmC);
+  }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc_cg<CG>(tmem_slot, TMEM_COLS);
+    tmem_relinquish_cg<CG>();
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if (CG == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_sync();   // set-up above overlapped the previous kernel's tail; operands are read from here on
@@ -210,119 +226,118 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     // warp-uniform loop, one elected lane issues (coordinates, addresses and the tensor-map pointers stay
-    // in uniform registers; the MN-major operands need up to six loads per k-block)
+    // in uniform registers). With CG = 2 every load of the pair is counted on the even CTA's barrier, whose CTA
+    // issues the products.
     const bool leader = elect_one();
-    if (leader) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
-    }
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int wi = 0; ok; ++wi) {
       TileInfo ti;
-      const int got = next_work<BN>(p, wi, num_tiles, num_kb, ti);
+      const int got = next_work<CG>(p, wi, num_tiles, num_kb, ti);
       if (got == 0) break;
       if (got == 2) continue;
-      const int m0 = ti.m0, n0 = ti.n0;
+      const int m0 = ti.m0 + cta * GEMM_BM, n0 = ti.n0 + cta * (BN / CG);
       for (int kb = 0; kb < ti.nkb; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_EMPTY));
         if (!ok) break;
-        uint8_t* sa = smem + stage * S::STAGE_BYTES;
-        uint8_t* sb = sa + S::A_BYTES;
+        uint8_t* sa = ring + stage * p.stage_bytes;
+        uint8_t* sb = sa + GEMM_A_BYTES;
         const int k0 = ti.k_begin + kb * GEMM_BK;
         if (leader) {
-          mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+          if (cta == 0) mbar_expect_tx(&full_bar[stage], p.stage_bytes * CG);
+          const uint32_t bar = CG == 2 ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
           if (!A_MN) {
-            tma_load_2d(sa, &tmA, &full_bar[stage], k0, m0);
+            tma_load_2d_cg<CG>(sa, &tmA, bar, k0, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < GEMM_BM / 64; ++c)
-              tma_load_2d(sa + c * 8192, &tmA, &full_bar[stage], m0 + c * 64, k0);
+            for (int c = 0; c < GEMM_BM / 64; ++c) tma_load_2d_cg<CG>(sa + c * 8192, &tmA, bar, m0 + c * 64, k0);
           }
           if (!B_MN) {
-            tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0 + ti.b_row_off);
+            tma_load_2d_cg<CG>(sb, &tmB, bar, k0, n0 + ti.b_row_off);
           } else {
-#pragma unroll
-            for (int c = 0; c < BN / 64; ++c)
-              tma_load_2d(sb + c * 8192, &tmB, &full_bar[stage], n0 + c * 64, k0 + ti.b_row_off);
+            for (int c = 0; c < p.b_chunks; ++c)
+              tma_load_2d_cg<CG>(sb + c * 8192, &tmB, bar, n0 + c * 64, k0 + ti.b_row_off);
           }
         }
         __syncwarp();
-        if (++stage == STAGES) {
+        if (++stage == stages) {
           stage = 0;
           phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------ MMA issuer (even CTA of a pair)
     // The whole warp walks the loop so that stage addresses, descriptors and counters stay warp-uniform
     // (a single-lane branch keeps them in per-thread registers and pays a move into the uniform registers
     // for every operand of every tcgen05.mma); one elected lane issues.
-    const bool leader = elect_one();
-    int stage = 0;
-    uint32_t phase = 0;
-    int it = 0;
-    bool ok = true;
-    // the descriptors of one k-block differ only in the address field: +(bytes >> 4) per 16-wide K step
-    const uint32_t a_step = static_cast<uint32_t>(p.a_kadv) >> 4, b_step = static_cast<uint32_t>(p.b_kadv) >> 4;
-    for (int wi = 0; ok; ++wi) {
-      TileInfo ti;
-      const int got = next_work<BN>(p, wi, num_tiles, num_kb, ti);
-      if (got == 0) break;
-      if (got == 2) continue;
-      const int as = it & 1;
-      const uint32_t aphase = (it >> 1) & 1;
-      ++it;
-      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[as], aphase ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_ACC_EMPTY));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + as * BN;
-      for (int kb = 0; kb < ti.nkb; ++kb) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, KWU_ERR_TIMEOUT_FULL));
+    if (cta == 0) {
+      const bool leader = elect_one();
+      int stage = 0;
+      uint32_t phase = 0;
+      int it = 0;
+      bool ok = true;
+      // the descriptors of one k-block differ only in the address field: +(bytes >> 4) per 16-wide K step
+      const uint32_t a_step = static_cast<uint32_t>(p.a_kadv) >> 4, b_step = static_cast<uint32_t>(p.b_kadv) >> 4;
+      for (int wi = 0; ok; ++wi) {
+        TileInfo ti;
+        const int got = next_work<CG>(p, wi, num_tiles, num_kb, ti);
+        if (got == 0) break;
+        if (got == 2) continue;
+        const int as = it & 1;
+        const uint32_t aphase = (it >> 1) & 1;
+        ++it;
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster<CG>(&acc_empty[as], aphase ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_ACC_EMPTY));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sa = smem_u32(smem + stage * S::STAGE_BYTES);
-        const uint64_t ad = make_smem_desc(sa, p.a_lbo, p.a_sbo, SWZ_128B);
-        const uint64_t bd = make_smem_desc(sa + S::A_BYTES, p.b_lbo, p.b_sbo, SWZ_128B);
-        const uint32_t acc0 = kb > 0 ? 1u : 0u;
-        if (leader) {
-          mma_f16_ss(d_tmem, ad, bd, p.idesc, acc0);
+        const uint32_t d_tmem = tmem_base + as * 256;
+        for (int kb = 0; kb < ti.nkb; ++kb) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, KWU_ERR_TIMEOUT_FULL));
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sa = smem_u32(ring + stage * p.stage_bytes);
+          const uint64_t ad = make_smem_desc(sa, p.a_lbo, p.a_sbo, SWZ_128B);
+          const uint64_t bd = make_smem_desc(sa + GEMM_A_BYTES, p.b_lbo, p.b_sbo, SWZ_128B);
+          const uint32_t acc0 = kb > 0 ? 1u : 0u;
+          if (leader) {
+            mma_f16_ss_cg<CG>(d_tmem, ad, bd, p.idesc, acc0);
 #pragma unroll
-          for (int k = 1; k < GEMM_BK / 16; ++k) mma_f16_ss(d_tmem, ad + k * a_step, bd + k * b_step, p.idesc, 1u);
-          tc_commit(&empty_bar[stage]);
+            for (int k = 1; k < GEMM_BK / 16; ++k) mma_f16_ss_cg<CG>(d_tmem, ad + k * a_step, bd + k * b_step, p.idesc, 1u);
+            tc_commit_cg<CG>(&empty_bar[stage]);
+          }
+          __syncwarp();
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
+        if (ok && leader) tc_commit_cg<CG>(&acc_full[as]);
         __syncwarp();
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
       }
-      if (ok && leader) tc_commit(&acc_full[as]);
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    int it = 0;
+    uint8_t* patch = out_area + (warp - 2) * 8192;
+    int it = 0, ob = 0;            // tiles done; output patch in use
     bool ok = true;
     for (int wi = 0; ok; ++wi) {
       TileInfo ti;
-      const int got = next_work<BN>(p, wi, num_tiles, num_kb, ti);
+      const int got = next_work<CG>(p, wi, num_tiles, num_kb, ti);
       if (got == 0) break;
       if (got == 2) continue;
       const int as = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       ++it;
-      const int m0 = ti.m0, n0 = ti.n0;
-      void* Cout = reinterpret_cast<uint8_t*>(Cbase) + ti.c_off * (p.out_fp32 ? 4 : 2);
+      const int m0 = ti.m0 + cta * GEMM_BM, n0 = ti.n0;
       ok = mbar_wait(&acc_full[as], aphase, abort_flag, p.status, KWU_ERR_TIMEOUT_ACC_FULL);
       ok = __all_sync(0xffffffffu, ok);  // the TMEM loads below are warp-collective
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + quarter * 32 + lane;
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * BN;
+      const int row0 = m0 + quarter * 32;      // first output row of this warp
+      const int row = row0 + lane;
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * 256;
       // per-row state of the cross-entropy epilogues
       float run_max = -INFINITY, run_sum = 0.f, tgt = 0.f;
       bool tgt_here = false;
@@ -336,14 +351,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           row_cy = p.coef_y[row];
         }
       }
+      const int ncols = min(BN, p.N - n0);     // columns of this tile that exist
+      const bool tma_rows = row0 < p.M;        // a warp whose rows all lie below the matrix stores nothing
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; c * 32 < ncols; ++c) {
         uint32_t r[32];
         tmem_ld_x32(t_row + c * 32, r);
         tmem_ld_wait();
         const int col0 = n0 + c * 32;
         if (EPI == EPI_LSE) {
-          if (row < p.M && col0 < p.N) {
+          if (row < p.M) {
             // the column bound and the label only matter in one chunk of a row each: handled outside the
             // per-element loops, which are a scale, a maximum, and one fused multiply-add + exp2 per logit
             if (col0 + 32 > p.N) {
@@ -377,142 +394,117 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             run_sum = run_sum * fast_exp2((run_max - nm) * 1.4426950408889634f) + ((c0 + c1) + (c2 + c3));
             run_max = nm;
           }
-        } else if (EPI == EPI_DLOGITS) {
-          if (row < p.M && col0 < p.N) {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(row) * p.ldc + col0;
-            float f[32];
-            {
-              // g = coef_p * exp2(acc * alpha * log2e - lse * log2e); the one-hot term is applied afterwards, in
-              // the one chunk of the row that holds the label
-              const float a2 = p.alpha * 1.4426950408889634f, nb = -row_lse * 1.4426950408889634f;
-              const uint64_t a2p = pack_f32x2(a2, a2), nbp = pack_f32x2(nb, nb), cpp = pack_f32x2(row_cp, row_cp);
+        } else {
+          float f[32];
+          if (EPI == EPI_DLOGITS) {
+            // g = coef_p * exp2(acc * alpha * log2e - lse * log2e); the one-hot term is applied afterwards, in
+            // the one chunk of the row that holds the label
+            const float a2 = p.alpha * 1.4426950408889634f, nb = -row_lse * 1.4426950408889634f;
+            const uint64_t a2p = pack_f32x2(a2, a2), nbp = pack_f32x2(nb, nb), cpp = pack_f32x2(row_cp, row_cp);
 #pragma unroll
-              for (int j = 0; j < 32; j += 2) {
-                float e0, e1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), a2p, nbp), e0, e1);
-                unpack_f32x2(mul_f32x2(pack_f32x2(fast_exp2(e0), fast_exp2(e1)), cpp), f[j], f[j + 1]);
-              }
-              if (label >= col0 && label < col0 + 32) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (col0 + j == label) f[j] -= row_cy;
-              }
+            for (int j = 0; j < 32; j += 2) {
+              float e0, e1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), a2p, nbp), e0, e1);
+              unpack_f32x2(mul_f32x2(pack_f32x2(fast_exp2(e0), fast_exp2(e1)), cpp), f[j], f[j + 1]);
             }
-            if (col0 + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 v;
-                v.x = pack_bf16(f[8 * j + 0], f[8 * j + 1]);
-                v.y = pack_bf16(f[8 * j + 2], f[8 * j + 3]);
-                v.z = pack_bf16(f[8 * j + 4], f[8 * j + 5]);
-                v.w = pack_bf16(f[8 * j + 6], f[8 * j + 7]);
-                reinterpret_cast<uint4*>(dst)[j] = v;
-              }
-            } else {
+            if (label >= col0 && label < col0 + 32) {
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (col0 + j < p.N) dst[j] = __float2bfloat16(f[j]);
-            }
-          }
-        } else if (p.out_fp32 && (p.splits > 1 || p.streamk > 0 || (p.group_mode == 2 && p.accumulate))) {
-          // Several CTAs add into the same tile (split-K, stream-K), or the tile is short in K and a
-          // read-modify-write would leave the epilogue waiting on loads (per-expert weight gradients):
-          // fire-and-forget vector reductions. The accumulator has one row per lane; the patch goes through
-          // shared memory so that the lanes of one reduction instruction cover whole 128-byte row segments.
-          if (col0 < p.N) {   // warp-uniform
-            float* stg = red_stage + (warp - 2) * (32 * 36);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<float4*>(stg + lane * 36 + 4 * j) =
-                  make_float4(__uint_as_float(r[4 * j]) * p.alpha, __uint_as_float(r[4 * j + 1]) * p.alpha,
-                              __uint_as_float(r[4 * j + 2]) * p.alpha, __uint_as_float(r[4 * j + 3]) * p.alpha);
-            __syncwarp();
-            const int c4 = (lane & 7) * 4;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int rr = i * 4 + (lane >> 3);
-              const int grow = m0 + quarter * 32 + rr;
-              const float4 v = *reinterpret_cast<const float4*>(stg + rr * 36 + c4);
-              if (grow < p.M) {
-                float* dst = reinterpret_cast<float*>(Cout) + static_cast<size_t>(grow) * p.ldc + col0 + c4;
-                if (col0 + c4 + 4 <= p.N) {
-                  red_add_f32x4(dst, v.x, v.y, v.z, v.w);
-                } else {
-                  const float f[4] = {v.x, v.y, v.z, v.w};
-                  for (int e = 0; e < 4; ++e)
-                    if (col0 + c4 + e < p.N) atomicAdd(dst + e, f[e]);
-                }
-              }
-            }
-            __syncwarp();
-          }
-        } else if (row < p.M && col0 < p.N) {
-          const bool full = (col0 + 32 <= p.N);
-          if (p.out_fp32) {
-            float* dst = reinterpret_cast<float*>(Cout) + static_cast<size_t>(row) * p.ldc + col0;
-            if (full) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                float4 v;
-                v.x = __uint_as_float(r[4 * j + 0]) * p.alpha;
-                v.y = __uint_as_float(r[4 * j + 1]) * p.alpha;
-                v.z = __uint_as_float(r[4 * j + 2]) * p.alpha;
-                v.w = __uint_as_float(r[4 * j + 3]) * p.alpha;
-                float4* d4 = reinterpret_cast<float4*>(dst) + j;
-                if (p.accumulate) {
-                  const float4 o = *d4;
-                  v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                *d4 = v;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (col0 + j < p.N) {
-                  float v = __uint_as_float(r[j]) * p.alpha;
-                  if (p.accumulate) v += dst[j];
-                  dst[j] = v;
-                }
-              }
+                if (col0 + j == label) f[j] -= row_cy;
             }
           } else {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(row) * p.ldc + col0;
-            if (p.row_ptrs) {
-              const long long base = p.row_ptrs[row];
-              if (!base) continue;
-              dst = reinterpret_cast<__nv_bfloat16*>(base) + col0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]) * p.alpha;
+          }
+          if (p.out_mode == OUT_TMA_BF16) {
+            // 64-column boxes: 128-byte rows, 16-byte units XORed with the row (the TMA's 128-byte swizzle);
+            // 32-column boxes: 64-byte rows, units XORed with row / 2 (its 64-byte swizzle). Conflict-free both ways.
+            const bool wide = p.out_cols == 64;
+            const bool first = !wide || (c & 1) == 0;      // first half of a box: the patch must be free again
+            if (first) {
+              if (lane == 0) tma_store_wait_read<1>();
+              __syncwarp();
             }
-            if (full) {
+            uint8_t* dst = patch + ob * 4096 + lane * (wide ? 128 : 64);
+            const int unit0 = wide ? (c & 1) * 4 : 0, key = wide ? (lane & 7) : ((lane >> 1) & 3);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]) * p.alpha;
-                uint4* d4 = reinterpret_cast<uint4*>(dst) + j;
-                if (p.accumulate) {
-                  const uint4 o = *d4;
-                  const float2 o0 = unpack_bf16(o.x), o1 = unpack_bf16(o.y), o2 = unpack_bf16(o.z),
-                               o3 = unpack_bf16(o.w);
-                  f[0] += o0.x; f[1] += o0.y; f[2] += o1.x; f[3] += o1.y;
-                  f[4] += o2.x; f[5] += o2.y; f[6] += o3.x; f[7] += o3.y;
-                }
-                uint4 v;
-                v.x = pack_bf16(f[0], f[1]);
-                v.y = pack_bf16(f[2], f[3]);
-                v.z = pack_bf16(f[4], f[5]);
-                v.w = pack_bf16(f[6], f[7]);
-                *d4 = v;
+            for (int j = 0; j < 4; ++j) {
+              uint4 v;
+              v.x = pack_bf16(f[8 * j + 0], f[8 * j + 1]);
+              v.y = pack_bf16(f[8 * j + 2], f[8 * j + 3]);
+              v.z = pack_bf16(f[8 * j + 4], f[8 * j + 5]);
+              v.w = pack_bf16(f[8 * j + 6], f[8 * j + 7]);
+              *reinterpret_cast<uint4*>(dst + (((unit0 + j) ^ key) << 4)) = v;
+            }
+            if (!wide || (c & 1) || (c + 1) * 32 >= ncols) {   // box complete (a last half box is cut at N by the TMA)
+              fence_async_proxy();
+              __syncwarp();
+              if (lane == 0 && tma_rows) {
+                tma_store_2d(&tmC, patch + ob * 4096, wide ? n0 + (c & ~1) * 32 : col0, row0 + ti.c_row_off);
+                tma_store_commit();
               }
-            } else {
+              ob ^= 1;
+            }
+          } else if (p.out_mode == OUT_TMA_F32 || p.out_mode == OUT_TMA_ADD) {
+            if (lane == 0) tma_store_wait_read<1>();
+            __syncwarp();
+            uint8_t* dst = patch + ob * 4096 + lane * 128;
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (col0 + j < p.N) {
-                  float v = __uint_as_float(r[j]) * p.alpha;
-                  if (p.accumulate) v += __bfloat162float(dst[j]);
-                  dst[j] = __float2bfloat16(v);
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(dst + ((j ^ (lane & 7)) << 4)) = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+            fence_async_proxy();
+            __syncwarp();
+            if (lane == 0 && tma_rows) {
+              if (p.out_mode == OUT_TMA_ADD)
+                tma_reduce_add_2d(&tmC, patch + ob * 4096, col0, row0 + ti.c_row_off);
+              else
+                tma_store_2d(&tmC, patch + ob * 4096, col0, row0 + ti.c_row_off);
+              tma_store_commit();
+            }
+            ob ^= 1;
+          } else if (row < p.M) {
+            const int valid = min(32, p.N - col0);
+            const size_t at = static_cast<size_t>(row + ti.c_row_off) * p.ldc + col0;
+            if (p.out_fp32) {
+              float* dst = reinterpret_cast<float*>(Cbase) + at;
+              // several CTAs may add into one element (split tail)
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (j < valid) {
+                  if (p.accumulate) atomicAdd(dst + j, f[j]); else dst[j] = f[j];
                 }
+            } else {
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(Cbase) + at;
+              bool vec = valid == 32 && (p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(Cbase) & 15) == 0;
+              bool drop = false;
+              if (p.row_ptrs) {
+                const long long base = p.row_ptrs[row];
+                drop = base == 0;
+                dst = reinterpret_cast<__nv_bfloat16*>(base) + col0;
+                vec = valid == 32 && (base & 15) == 0;
+              }
+              if (!drop && vec) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  float* g = f + 8 * j;
+                  uint4* d4 = reinterpret_cast<uint4*>(dst) + j;
+                  if (p.accumulate) {
+                    const uint4 o = *d4;
+                    const float2 o0 = unpack_bf16(o.x), o1 = unpack_bf16(o.y), o2 = unpack_bf16(o.z), o3 = unpack_bf16(o.w);
+                    g[0] += o0.x; g[1] += o0.y; g[2] += o1.x; g[3] += o1.y;
+                    g[4] += o2.x; g[5] += o2.y; g[6] += o3.x; g[7] += o3.y;
+                  }
+                  uint4 v;
+                  v.x = pack_bf16(g[0], g[1]);
+                  v.y = pack_bf16(g[2], g[3]);
+                  v.z = pack_bf16(g[4], g[5]);
+                  v.w = pack_bf16(g[6], g[7]);
+                  *d4 = v;
+                }
+              } else if (!drop) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (j < valid) dst[j] = __float2bfloat16(p.accumulate ? f[j] + __bfloat162float(dst[j]) : f[j]);
               }
             }
           }
@@ -523,8 +515,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (tgt_here) p.target_logit[row] = tgt;
       }
       tc_fence_before();
-      mbar_arrive(&acc_empty[as]);
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[as]), 0));
+        else mbar_arrive(&acc_empty[as]);
+      }
     }
+    if (lane == 0) tma_store_wait_read<0>();   // the patches are read before this CTA's shared memory goes away
   }
 
   // ---------------------------------------------------------------- tear-down
@@ -534,29 +531,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // give copies that are still in flight time to land before the CTA's smem goes away
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }
+  if (CG == 2) cluster_sync();   // the pair leaves together: its barriers and TMEM are used from both sides
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc_cg<CG>(tmem_base, TMEM_COLS);
   }
 }
 
 // ------------------------------------------------------------------ host launcher
-static int g_num_sms = 0;
 static int num_sms() {
-  if (!g_num_sms) {
-    int dev = 0;
+  static int n = 0;
+  if (!n) {
+    int dev = 0, v = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0) g_num_sms = 148;
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n = v > 0 ? v : 148;
   }
-  return g_num_sms;
+  return n;
 }
-
-struct DescOverride {
-  int active = 0;
-  uint32_t a_lbo, a_sbo, a_kadv, b_lbo, b_sbo, b_kadv;
-};
-static DescOverride g_override;
 
 struct GroupArgs {
   int mode = 0;
@@ -564,7 +556,7 @@ struct GroupArgs {
   const int* offsets = nullptr;
   int b_rows = 0;
   int num_groups = 1;
-  long long c_stride = 0;
+  int c_rows = 0;
   int row_tiles = 0;  // mode 1: number of entries in `tiles`
   const long long* row_ptrs = nullptr;
 };
@@ -578,13 +570,12 @@ struct EpiArgs {
   const float* coef_y = nullptr;
 };
 
-template <int BN, bool A_MN, bool B_MN, int EPI = EPI_STORE>
-static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
+template <int CG, bool A_MN, bool B_MN, int EPI>
+static int launch_gemm(int BN, const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                        int ldc, int out_fp32, int accumulate, float alpha, int max_ctas,
                        cudaStream_t stream, int* status, const EpiArgs& ea = EpiArgs(),
-                       const GroupArgs& ga = GroupArgs(), int b_total_rows = 0, int splits = 1, bool streamk = false) {
-  using S = GemmSmem<BN>;
-  CUtensorMap tmA, tmB;
+                       const GroupArgs& ga = GroupArgs(), int b_total_rows = 0, int splits = 1) {
+  CUtensorMap tmA, tmB, tmC;
   int rc;
   if (!A_MN)
     rc = encode_tmap_2d(&tmA, A, ELEM_BF16, M, K, lda, GEMM_BM, GEMM_BK, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -593,57 +584,79 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (rc) return rc;
   // with expert groups B is the stack of all experts' matrices: b_total_rows rows in storage order
   if (!B_MN)
-    rc = encode_tmap_2d(&tmB, B, ELEM_BF16, b_total_rows ? b_total_rows : N, K, ldb, BN, GEMM_BK, CU_TENSOR_MAP_SWIZZLE_128B);
+    rc = encode_tmap_2d(&tmB, B, ELEM_BF16, b_total_rows ? b_total_rows : N, K, ldb, BN / CG, GEMM_BK, CU_TENSOR_MAP_SWIZZLE_128B);
   else
     rc = encode_tmap_2d(&tmB, B, ELEM_BF16, b_total_rows ? b_total_rows : K, N, ldb, GEMM_BK, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
 
   GemmParams p;
-  p.M = M; p.N = N; p.K = K; p.ldc = ldc;
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.bn = BN;
   p.out_fp32 = out_fp32; p.accumulate = accumulate; p.alpha = alpha;
   // K-major, 128B swizzle: rows are 128 B, 8-row groups 1024 B apart, K advances 32 B per MMA.
   // MN-major, 128B swizzle: 64-element chunks along MN are whole 8 KB boxes, 8-row K groups are
   // 1024 B apart, K advances 16 rows = 2048 B per MMA.
   p.a_lbo = A_MN ? 8192 : 16; p.a_sbo = 1024; p.a_kadv = A_MN ? 2048 : 32;
   p.b_lbo = B_MN ? 8192 : 16; p.b_sbo = 1024; p.b_kadv = B_MN ? 2048 : 32;
-  if (g_override.active) {
-    if (A_MN) { p.a_lbo = g_override.a_lbo; p.a_sbo = g_override.a_sbo; p.a_kadv = g_override.a_kadv; }
-    if (B_MN) { p.b_lbo = g_override.b_lbo; p.b_sbo = g_override.b_sbo; p.b_kadv = g_override.b_kadv; }
-  }
-  p.idesc = make_idesc_f16(GEMM_BM, BN, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
-  p.tiles_m = ga.mode == 1 ? ga.row_tiles : (M + GEMM_BM - 1) / GEMM_BM;
+  p.idesc = make_idesc_f16(GEMM_BM * CG, BN, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
+  p.b_chunks = (BN / CG + 63) / 64;
+  p.stage_bytes = GEMM_A_BYTES + (B_MN ? p.b_chunks * 64 : BN / CG) * GEMM_BK * 2;
+  p.stages = (GEMM_SMEM_MAX - 1024 - GEMM_BAR_BYTES - GEMM_OUT_BYTES) / static_cast<int>(p.stage_bytes);
+  if (p.stages > GEMM_MAX_STAGES) p.stages = GEMM_MAX_STAGES;
+  p.tiles_m = ga.mode == 1 ? ga.row_tiles : (M + GEMM_BM * CG - 1) / (GEMM_BM * CG);
   p.tiles_n = (N + BN - 1) / BN;
   p.status = status;
-  p.splits = (ga.mode == 0 && out_fp32 && accumulate) ? splits : 1;
-  p.streamk = 0;
   p.group_mode = ga.mode; p.group_tiles = ga.tiles; p.group_offsets = ga.offsets;
-  p.group_b_rows = ga.b_rows; p.num_groups = ga.num_groups; p.c_group_stride = ga.c_stride;
+  p.group_b_rows = ga.b_rows; p.num_groups = ga.num_groups; p.c_group_rows = ga.c_rows;
   p.row_ptrs = (EPI == EPI_STORE && !out_fp32) ? ga.row_ptrs : nullptr;
   p.labels = ea.labels; p.partial = ea.partial; p.target_logit = ea.target_logit;
   p.lse = ea.lse; p.coef_p = ea.coef_p; p.coef_y = ea.coef_y;
 
-  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, EPI>;
+  // TMA addresses the output when its base and pitch are 16-byte multiples; rows of one expert's gradient must fill
+  // whole tiles, or the store box would reach into the next expert's rows
+  const bool can_tma = EPI != EPI_LSE && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * (out_fp32 ? 4 : 2)) % 16 == 0 &&
+                       !p.row_ptrs && (ga.mode != 2 || M % (GEMM_BM * CG) == 0);
+  p.out_mode = OUT_DIRECT;
+  p.out_cols = (BN % 64) ? 32 : 64;
+  if (can_tma && (out_fp32 || !accumulate))
+    p.out_mode = out_fp32 ? (accumulate ? OUT_TMA_ADD : OUT_TMA_F32) : OUT_TMA_BF16;
+  if (p.out_mode != OUT_DIRECT) {
+    const uint64_t c_rows = ga.mode == 2 ? static_cast<uint64_t>(ga.num_groups) * ga.c_rows : M;
+    if (out_fp32)
+      rc = encode_tmap_2d(&tmC, C, ELEM_F32, c_rows, N, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B);
+    else
+      rc = encode_tmap_2d(&tmC, C, ELEM_BF16, c_rows, N, ldc, 32, p.out_cols,
+                          p.out_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc) return rc;
+  } else {
+    tmC = tmA;   // not read
+  }
+
+  auto kern = gemm_bf16_kernel<CG, A_MN, B_MN, EPI>;
   static PerDeviceOnce attr_set;
   if (attr_set.pending()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_MAX);
     if (e != cudaSuccess) {
       set_last_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return 10;
     }
     attr_set.mark();
   }
-  long grid_l = static_cast<long>(p.tiles_m) * p.tiles_n * (ga.mode == 2 ? ga.num_groups : 1) * (p.splits > 1 ? p.splits : 1);
-  int grid = grid_l > (1 << 30) ? (1 << 30) : static_cast<int>(grid_l);
-  int cap = num_sms();
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
-  if (grid > cap) grid = cap;
-  if (streamk && ga.mode == 0 && out_fp32 && accumulate && EPI == EPI_STORE) {
-    const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * ((K + GEMM_BK - 1) / GEMM_BK);
-    grid = static_cast<int>(units < cap ? units : cap);
-    p.splits = 1;
-    p.streamk = grid;
+  long tiles = static_cast<long>(p.tiles_m) * p.tiles_n * (ga.mode == 2 ? ga.num_groups : 1);
+  int units = num_sms();
+  if (max_ctas > 0 && max_ctas < units) units = max_ctas;
+  units = units / CG > 0 ? units / CG : 1;
+  p.full_tiles = static_cast<int>(tiles);
+  p.tail_tiles = 0;
+  p.splits = 1;
+  if (splits > 1 && ga.mode == 0 && out_fp32 && accumulate && EPI == EPI_STORE) {
+    p.full_tiles = static_cast<int>(tiles - tiles % units);
+    p.tail_tiles = static_cast<int>(tiles % units);
+    p.splits = splits;
   }
-  launch_k(kern, dim3(grid), dim3(GEMM_THREADS), S::TOTAL, stream, tmA, tmB, C, p); kwu::count_launch();
+  const long items = p.full_tiles + static_cast<long>(p.tail_tiles) * p.splits;
+  if (items < units) units = static_cast<int>(items);
+  const size_t smem = 1024 + GEMM_BAR_BYTES + GEMM_OUT_BYTES + static_cast<size_t>(p.stages) * p.stage_bytes;
+  launch_cluster(kern, dim3(units * CG), dim3(GEMM_THREADS), CG, smem, stream, tmA, tmB, tmC, C, p); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_error("gemm launch: %s", cudaGetErrorString(e));
@@ -652,60 +665,75 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   return 0;
 }
 
-static int pick_bn(int M, int N, int forced) {
-  if (forced == 128 || forced == 256) return forced;
-  const int sms = num_sms();
-  const int tm = (M + GEMM_BM - 1) / GEMM_BM;
-  const long t256 = static_cast<long>(tm) * ((N + 255) / 256);
-  const long t128 = static_cast<long>(tm) * ((N + 127) / 128);
-  const long c256 = ((t256 + sms - 1) / sms) * 256;
-  const long c128 = ((t128 + sms - 1) / sms) * 128;
-  // a wide tile re-reads A half as often; prefer it unless the narrow one saves a real wave
-  return (c128 * 100 < c256 * 92) ? 128 : 256;
+struct TilePick {
+  int cg, bn, splits;
+};
+
+// Tile (one CTA or a pair, width) and split of the tail round with the least predicted time. Measured on one B200
+// (8192^3, 4096 x 7168 x 1280, 16384 x 1536 x 8192 and 2560 x 1536 x 16384, operands rotating through four buffers): a
+// 64-deep k-block takes a pair 0.070 us + 1.25 ns per column with B K-major, 0.25 us + 0.47 ns with B MN-major (its
+// boxes are 64 columns of each CTA whatever the width), and a single CTA 0.19 us + 0.9 ns; every round of the
+// persistent grid takes another 0.55 us (accumulator hand-over, pipeline refill). The rounds decide
+// between widths: 4096 x 1280 is two rounds of 160 columns or two of 256. fp32 C += may cut the tiles of its last,
+// partly empty round along the contraction (no cut below 4 k-blocks).
+static TilePick pick_tile(int M, int N, int K, bool b_mn, bool can_split, int tiles_m128 = 0, int max_cg = 2, int max_ctas = 0) {
+  int sms = num_sms();
+  if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
+  const int nkb = (K + GEMM_BK - 1) / GEMM_BK;
+  TilePick best{1, 128, 1};
+  double best_cost = 1e30;
+  for (int cg = 1; cg <= max_cg; ++cg) {
+    if (cg == 2 && (M <= GEMM_BM || sms < 2)) continue;
+    const long tm = tiles_m128 ? tiles_m128 : (M + GEMM_BM * cg - 1) / (GEMM_BM * cg);
+    const int units = sms / cg;
+    for (int bn = cg == 1 ? 64 : 128; bn <= 256; bn += 32) {
+      const long tiles = tm * ((N + bn - 1) / bn);
+      const double per_kb = cg == 1 ? 0.19 + 0.0009 * bn : (b_mn ? 0.25 + 0.00047 * bn : 0.070 + 0.00125 * bn);
+      const long full = tiles / units, tail = tiles % units;
+      double cost = full * (nkb * per_kb + 0.55);
+      int splits = 1;
+      if (tail > 0) {
+        if (can_split) {
+          splits = static_cast<int>(units / tail);
+          if (splits > nkb / 4) splits = nkb / 4;
+          if (splits < 1) splits = 1;
+        }
+        cost += (nkb + splits - 1) / splits * per_kb + 0.55;
+      }
+      if (cost < best_cost - 1e-9) { best_cost = cost; best = {cg, bn, splits}; }
+    }
+  }
+  return best;
 }
 
 }  // namespace kwu
 
 // C[M,N] (+)= alpha * op(A) op(B). a_mn / b_mn select the storage described at the top of the file.
-// lda/ldb/ldc are row pitches in elements of the STORED matrices. bn: 0 = choose, 128 or 256.
+// lda/ldb/ldc are row pitches in elements of the STORED matrices. bn: 0 = choose, 64..256 = a tile of one CTA that
+// wide (multiples of 32), 1000 + width = a tile of a CTA pair.
 KWU_API int kwu_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                           int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, float alpha,
                           int bn, int max_ctas, void* stream, int* status) {
   using namespace kwu;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int BN = pick_bn(M, N, bn);
-  int splits = 1;
-  bool streamk = false;
-  if (out_fp32 && accumulate && bn == 0 && K >= 1024) {
-    // weight-gradient shape: few output tiles, long contraction, C += semantics. Wide tiles, and the
-    // (tile, k-block) units are dealt out evenly over the SMs (stream-K) unless the tiles already fill
-    // whole waves.
-    const int sms = num_sms();
-    const long t256 = static_cast<long>((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256);
-    BN = 256;
-    streamk = (t256 % sms) != 0;
+  TilePick pick{bn > 1000 ? 2 : 1, bn > 1000 ? bn - 1000 : bn, 1};
+  if (bn == 0) pick = pick_tile(M, N, K, b_mn != 0, out_fp32 && accumulate, 0, 2, max_ctas);
+  if (pick.bn < 64 || pick.bn > 256 || pick.bn % 32) {
+    set_last_error("kwu_gemm_bf16: tile width %d", pick.bn);
+    return 20;
   }
-#define KWU_GEMM_CASE(bnv, amn, bmn)                                                              \
-  if (BN == bnv && a_mn == amn && b_mn == bmn)                                                    \
-    return launch_gemm<bnv, amn != 0, bmn != 0>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32,        \
+#define KWU_GEMM_CASE(cgv, amn, bmn)                                                              \
+  if (pick.cg == cgv && a_mn == amn && b_mn == bmn)                                               \
+    return launch_gemm<cgv, amn != 0, bmn != 0, EPI_STORE>(pick.bn, A, B, C, M, N, K, lda, ldb, ldc, out_fp32,        \
                                                 accumulate, alpha, max_ctas, st, status, EpiArgs(), \
-                                                GroupArgs(), 0, splits, streamk);
-  KWU_GEMM_CASE(128, 0, 0) KWU_GEMM_CASE(128, 0, 1) KWU_GEMM_CASE(128, 1, 0) KWU_GEMM_CASE(128, 1, 1)
-  KWU_GEMM_CASE(256, 0, 0) KWU_GEMM_CASE(256, 0, 1) KWU_GEMM_CASE(256, 1, 0) KWU_GEMM_CASE(256, 1, 1)
+                                                GroupArgs(), 0, pick.splits);
+  KWU_GEMM_CASE(1, 0, 0) KWU_GEMM_CASE(1, 0, 1) KWU_GEMM_CASE(1, 1, 0) KWU_GEMM_CASE(1, 1, 1)
+  KWU_GEMM_CASE(2, 0, 0) KWU_GEMM_CASE(2, 0, 1) KWU_GEMM_CASE(2, 1, 0) KWU_GEMM_CASE(2, 1, 1)
 #undef KWU_GEMM_CASE
   set_last_error("kwu_gemm_bf16: unsupported variant");
   return 20;
 }
-
-// Test hook: override the MN-major descriptor constants (used once to pin the layout rules).
-KWU_API void kwu_gemm_debug_override(int active, unsigned a_lbo, unsigned a_sbo, unsigned a_kadv,
-                                     unsigned b_lbo, unsigned b_sbo, unsigned b_kadv) {
-  kwu::g_override.active = active;
-  kwu::g_override.a_lbo = a_lbo; kwu::g_override.a_sbo = a_sbo; kwu::g_override.a_kadv = a_kadv;
-  kwu::g_override.b_lbo = b_lbo; kwu::g_override.b_sbo = b_sbo; kwu::g_override.b_kadv = b_kadv;
-}
-
 
 // ------------------------------------------------------------------ fused linear cross-entropy
 // Forward: logits = alpha * h W^T are never written. Every (row, 256-column tile) leaves one
@@ -722,8 +750,12 @@ KWU_API int kwu_gemm_lse(const void* H, const void* W, int T, int V, int D, int 
   ea.labels = labels;
   ea.partial = reinterpret_cast<float2*>(partial);
   ea.target_logit = target_logit;
-  return launch_gemm<256, false, false, EPI_LSE>(H, W, nullptr, T, V, D, ldh, ldw, 0, 0, 0, alpha, 0,
+  // the partial table has one column per 256 logits, so the width is fixed
+  if (T > GEMM_BM)
+    return launch_gemm<2, false, false, EPI_LSE>(256, H, W, nullptr, T, V, D, ldh, ldw, 0, 0, 0, alpha, 0,
                                                  reinterpret_cast<cudaStream_t>(stream), status, ea);
+  return launch_gemm<1, false, false, EPI_LSE>(256, H, W, nullptr, T, V, D, ldh, ldw, 0, 0, 0, alpha, 0,
+                                               reinterpret_cast<cudaStream_t>(stream), status, ea);
 }
 
 // Backward recompute: dlogits[row, col] = coef_p[row] * exp(logit - lse[row]) - coef_y[row] * onehot,
@@ -739,8 +771,11 @@ KWU_API int kwu_gemm_dlogits(const void* H, const void* W, void* dlogits, int T,
   ea.lse = lse;
   ea.coef_p = coef_p;
   ea.coef_y = coef_y;
-  return launch_gemm<256, false, false, EPI_DLOGITS>(H, W, dlogits, T, V, D, ldh, ldw, ldd, 0, 0, alpha,
+  if (T > GEMM_BM)
+    return launch_gemm<2, false, false, EPI_DLOGITS>(256, H, W, dlogits, T, V, D, ldh, ldw, ldd, 0, 0, alpha,
                                                      0, reinterpret_cast<cudaStream_t>(stream), status, ea);
+  return launch_gemm<1, false, false, EPI_DLOGITS>(256, H, W, dlogits, T, V, D, ldh, ldw, ldd, 0, 0, alpha,
+                                                   0, reinterpret_cast<cudaStream_t>(stream), status, ea);
 }
 
 namespace kwu {
@@ -790,10 +825,12 @@ KWU_API int kwu_gemm_bf16_grouped_rows(const void* A, const void* B, void* C, in
   ga.b_rows = b_mn ? K : N;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int total_rows = num_experts * ga.b_rows;
+  // tiles stay inside one expert's 128-aligned rows, so a single CTA each
+  const int bn = pick_tile(M_pad, N, K, b_mn != 0, false, row_tiles, 1).bn;
   if (b_mn)
-    return launch_gemm<128, false, true>(A, B, C, M_pad, N, K, lda, ldb, ldc, out_fp32, 0, 1.f, 0, st, status,
+    return launch_gemm<1, false, true, EPI_STORE>(bn, A, B, C, M_pad, N, K, lda, ldb, ldc, out_fp32, 0, 1.f, 0, st, status,
                                          EpiArgs(), ga, total_rows);
-  return launch_gemm<128, false, false>(A, B, C, M_pad, N, K, lda, ldb, ldc, out_fp32, 0, 1.f, 0, st, status,
+  return launch_gemm<1, false, false, EPI_STORE>(bn, A, B, C, M_pad, N, K, lda, ldb, ldc, out_fp32, 0, 1.f, 0, st, status,
                                         EpiArgs(), ga, total_rows);
 }
 
@@ -803,12 +840,20 @@ KWU_API int kwu_gemm_bf16_grouped_wgrad(const void* dY, const void* X, void* dW,
                                         int lddy, int ldx, int num_experts, const int* offsets, int out_fp32,
                                         int accumulate, void* stream, int* status) {
   using namespace kwu;
-  if (M_pad <= 0) return 0;
+  if (M_pad <= 0 || num_experts <= 0) return 0;
   GroupArgs ga;
   ga.mode = 2;
   ga.offsets = offsets;
   ga.num_groups = num_experts;
-  ga.c_stride = static_cast<long long>(N_out) * K_out;
-  return launch_gemm<128, true, true>(dY, X, dW, N_out, K_out, M_pad, lddy, ldx, K_out, out_fp32, accumulate, 1.f,
-                                      0, reinterpret_cast<cudaStream_t>(stream), status, EpiArgs(), ga, 0);
+  ga.c_rows = N_out;
+  // a pair's 256 rows must not reach into the next expert's gradient
+  const int cgs = N_out % (2 * GEMM_BM) == 0 ? 2 : 1;
+  const int rows = (N_out + GEMM_BM - 1) / GEMM_BM * GEMM_BM * num_experts;
+  const TilePick pick = pick_tile(rows, K_out, M_pad / num_experts + GEMM_BK, true, false, 0, cgs);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (pick.cg == 2)
+    return launch_gemm<2, true, true, EPI_STORE>(pick.bn, dY, X, dW, N_out, K_out, M_pad, lddy, ldx, K_out, out_fp32,
+                                                 accumulate, 1.f, 0, st, status, EpiArgs(), ga, 0);
+  return launch_gemm<1, true, true, EPI_STORE>(pick.bn, dY, X, dW, N_out, K_out, M_pad, lddy, ldx, K_out, out_fp32,
+                                               accumulate, 1.f, 0, st, status, EpiArgs(), ga, 0);
 }

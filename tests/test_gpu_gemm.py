@@ -76,3 +76,27 @@ def test_stream_k_weight_gradient_accumulates_exactly_once(M, N, K):
     torch.cuda.synchronize()
     native.check_status()
     torch.testing.assert_close(out, ref + 2.0, rtol=1e-4, atol=2e-3 * (K / 4096) ** 0.5 + 1e-3)
+
+
+@pytest.mark.parametrize("bn", [64, 96, 160, 224, 1128, 1160, 1192, 1224, 1256])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("shape", [(136, 72, 72), (264, 328, 200), (520, 1064, 136)])
+def test_gemm_tile_widths_and_cta_pairs(shape, a_mn, b_mn, bn):
+    """Every tile width of one CTA and of a CTA pair (1000 + width), rows and columns that end inside a tile, a pair whose
+    second CTA has few or no rows, a contraction that ends inside a k-block; bf16 store, fp32 store and fp32 C +=. The
+    row of canaries behind the output must survive: a store box that is not cut at the edge would write there."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.gemm import matmul
+
+    M, N, K = shape
+    a, b, ref = _operands(M, N, K, a_mn, b_mn, seed=bn)
+    for dtype, acc in ((torch.bfloat16, False), (torch.float32, False), (torch.float32, True)):
+        full = torch.full((M + 1, N), 3.0, device="cuda", dtype=dtype)
+        matmul(a, b, a_mn=a_mn, b_mn=b_mn, out=full[:M], accumulate=acc, bn=bn)
+        torch.cuda.synchronize()
+        native.check_status()
+        want = ref + 3.0 if acc else ref
+        # bf16: half a unit in the last place (2^-9); fp32: the order of K <= 200 sums (K * 2^-24, scaled by the largest value)
+        tol = 2.0 ** -8 if dtype == torch.bfloat16 else 200 * 2.0 ** -23
+        assert (full[:M].float() - want).abs().max().item() <= tol * want.abs().max().item()
+        assert bool((full[M] == 3.0).all())
