@@ -779,24 +779,44 @@ KWU_API int kwu_gemm_dlogits(const void* H, const void* W, void* dlogits, int T,
 }
 
 namespace kwu {
-__global__ void ce_combine_kernel(const float2* __restrict__ partial, int tiles_n, int M,
-                                  float* __restrict__ lse) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= M) return;
+// 32 rows by 8 slices of the column tiles per block: a thread folds every eighth partial of its row (a warp reads 256
+// contiguous bytes), then the slices are folded in shared memory. One thread per row alone left 64 of 148 SMs with
+// one chain of 256 dependent loads each (40 us at 8190 rows and 256 tiles; 6 us like this).
+constexpr int CE_ROWS = 32, CE_SLICES = 8;
+__global__ void __launch_bounds__(CE_ROWS * CE_SLICES) ce_combine_kernel(const float2* __restrict__ partial, int tiles_n, int M,
+                                                                         float* __restrict__ lse) {
+  __shared__ float2 part[CE_SLICES][CE_ROWS];
+  const int r = threadIdx.x % CE_ROWS, sl = threadIdx.x / CE_ROWS;
+  const int row = blockIdx.x * CE_ROWS + r;
   float m = -INFINITY, s = 0.f;
-  for (int t = 0; t < tiles_n; ++t) {
-    const float2 v = partial[static_cast<size_t>(t) * M + row];
-    const float nm = fmaxf(m, v.x);
-    s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
-    m = nm;
+  if (row < M) {
+    for (int t = sl; t < tiles_n; t += CE_SLICES) {
+      const float2 v = partial[static_cast<size_t>(t) * M + row];
+      const float nm = fmaxf(m, v.x);
+      s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
+      m = nm;
+    }
   }
-  lse[row] = m + __logf(s);
+  part[sl][r] = make_float2(m, s);
+  __syncthreads();
+  if (sl == 0 && row < M) {
+#pragma unroll
+    for (int i = 1; i < CE_SLICES; ++i) {
+      const float2 v = part[i][r];
+      if (v.x == -INFINITY) continue;      // a slice without a tile
+      const float nm = fmaxf(m, v.x);
+      s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
+      m = nm;
+    }
+    lse[row] = m + __logf(s);
+  }
 }
 }  // namespace kwu
 
 KWU_API int kwu_ce_combine(const void* partial, int tiles_n, int M, float* lse, void* stream) {
   if (M <= 0) return 0;
-  kwu::ce_combine_kernel<<<(M + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  kwu::ce_combine_kernel<<<(M + kwu::CE_ROWS - 1) / kwu::CE_ROWS, kwu::CE_ROWS * kwu::CE_SLICES, 0,
+                           reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const float2*>(partial), tiles_n, M, lse); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { kwu::set_last_error("ce_combine launch: %s", cudaGetErrorString(e)); return 11; }

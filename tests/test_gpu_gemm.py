@@ -100,3 +100,18 @@ def test_gemm_tile_widths_and_cta_pairs(shape, a_mn, b_mn, bn):
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 200 * 2.0 ** -23
         assert (full[:M].float() - want).abs().max().item() <= tol * want.abs().max().item()
         assert bool((full[M] == 3.0).all())
+
+
+@pytest.mark.parametrize("vocab", [1000, 256 * 9])
+def test_cross_entropy_partials_fold(vocab):
+    """Column tiles that do not fill the eight slices of the folding kernel, and rows that end inside its block."""
+    from kohakuwullm_b200.ops.loss import linear_cross_entropy, linear_cross_entropy_reference
+
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    h = torch.randn(133, 128, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(vocab, 128, device="cuda", generator=g) * 0.2).to(torch.bfloat16)
+    labels = torch.randint(0, vocab, (133,), device="cuda", generator=g)
+    ce, lse = linear_cross_entropy(h, w, labels)
+    want_ce, want_lse = linear_cross_entropy_reference(h, w, labels)
+    torch.testing.assert_close(lse, want_lse, rtol=1e-4, atol=1e-3)
+    torch.testing.assert_close(ce, want_ce, rtol=1e-4, atol=1e-3)
