@@ -424,6 +424,26 @@ __device__ __forceinline__ void mma_f16_ss_cg(uint32_t d_tmem, uint64_t a_desc, 
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+template <int CG>
+__device__ __forceinline__ void mma_mxf8_ss_cg(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem,
+                                               uint32_t sfb_tmem, uint32_t accumulate) {
+  if (CG == 1) return mma_mxf8_ss(d_tmem, a_desc, b_desc, idesc, sfa_tmem, sfb_tmem, accumulate);
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
+      : "memory");
+}
+// With CG = 2 each CTA's shared memory is copied into its own TMEM.
+template <int CG>
+__device__ __forceinline__ void tc_cp_32x128b_warpx4_cg(uint32_t taddr, uint64_t sdesc) {
+  if (CG == 1) return tc_cp_32x128b_warpx4(taddr, sdesc);
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
 // With CG = 2 the barrier at the same offset of BOTH CTAs gets the arrival.
 template <int CG>
 __device__ __forceinline__ void tc_commit_cg(uint64_t* bar) {

@@ -129,18 +129,23 @@ TILE_WIDTHS = (128, 144, 160, 176, 192, 208, 224, 240)
 def pick_tile_width(n_cols: int, m_rows: int = 4096, sms: int = 148) -> int:
     """Width of the output tiles of ``A (m_rows, K) x W (n_cols, K)^T`` that minimises rounds x cost per round.
 
-    The block-scaled GEMM is bound by shared-memory traffic: per 128-deep k-block a 128 x BN tile moves
-    16 KB + BN * 128 B, so a round of tiles costs ``16 + BN / 8`` units whatever it computes, and a problem
-    takes ``ceil(tiles / SMs)`` rounds. A wider tile is cheaper per column, and the right width fills whole
-    waves (4096 x 1280: 320 tiles of 128 are 3 rounds, 288 tiles of 144 are 2). ``KWU_MX_BN`` forces a width."""
+    Products of more than 128 rows run on pairs of SMs (256-row tiles, widths that are multiples of 32). A round of the
+    pairs costs ``108 + BN`` units, fitted to B200 times of 14 products of 2048 to 8192 rows and K 1024 to 7168 (at K =
+    1280: 3.1 us for 128 columns, 3.6 for 160, 3.9 for 192, 4.5 for 224), and a problem takes ``ceil(tiles / pairs)``
+    rounds: 4096 x 1280 is three rounds of 128 columns or two of 160 (27.2 and 20.9 us at K = 3584), 4096 x 7168
+    thirteen or seven of 224 (43.4 and 34.9 us at K = 1280). Fewer rows are one CTA's tiles, bound by shared-memory
+    traffic of 16 KB + BN * 128 B per 128-deep k-block: ``16 + BN / 8``. ``KWU_MX_BN`` forces a width."""
     forced = os.environ.get("KWU_MX_BN")
     if forced:
         return int(forced)
-    tiles_m = max((m_rows + 127) // 128, 1)
+    pairs = m_rows > 128
+    tiles_m = max((m_rows + 255) // 256 if pairs else (m_rows + 127) // 128, 1)
     best, best_bn = None, 128
     for bn in TILE_WIDTHS:
-        rounds = -(-(tiles_m * -(-n_cols // bn)) // sms)
-        cost = rounds * (16 + bn / 8)
+        if pairs and bn % 32:
+            continue
+        rounds = -(-(tiles_m * -(-n_cols // bn)) // (max(sms // 2, 1) if pairs else sms))
+        cost = rounds * (108 + bn if pairs else 16 + bn / 8)
         if best is None or cost < best - 1e-9:
             best, best_bn = cost, bn
     return best_bn

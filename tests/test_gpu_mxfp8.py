@@ -225,3 +225,35 @@ def test_own_mxfp8_gemm_agrees_with_the_vendor_library_on_the_same_bytes():
         assert r["ours_vs_vendor_max_ulp"] <= 1.0, r
         assert r["bit_equal_share"] >= 0.99, r
         assert r["ours_vs_fp64_max_ulp"] <= 2.0 and r["vendor_vs_fp64_max_ulp"] <= 2.0, r
+
+
+@pytest.mark.parametrize("bn", [128, 144, 160, 192, 224, 240])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (128, 256, 256), (129, 1280, 384), (640, 1168, 1280), (1000, 200, 512)])
+def test_gemm_tile_widths_and_outputs(M, N, K, bn):
+    """One CTA and pairs of CTAs, whole and cut tiles in both directions, each way the result leaves the kernel. The
+    oracle multiplies the dequantised operands in 64 bits. Bound: products of e4m3 values are exact in fp32, so an fp32
+    sum of K of them is off by at most K * 2^-24 of the sum of magnitudes (twice that for sums that truncate); a bf16
+    result by another 2^-9 of itself."""
+    from kohakuwullm_b200.ops import mxfp8 as mx, native
+
+    torch.manual_seed(M + bn)
+    a = (torch.randn(M, K, device="cuda") * torch.logspace(-2, 1, K, device="cuda")).to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda") * torch.logspace(1, -1, N, device="cuda")[:, None]).to(torch.bfloat16)
+    aq, asf = mx.quantize(a)
+    bq, bsf_plain = mx.quantize(b)
+    bsf = mx.alloc_weight_sf(N, K, bn, "cuda")
+    mx.quantize_weight(b, torch.empty_like(bq), bsf, bn)
+    da = mx.dequantize(aq.view(torch.float8_e4m3fn), mx.sf_to_natural(asf, M, K)).double()
+    db = mx.dequantize(bq.view(torch.float8_e4m3fn), mx.sf_to_natural(bsf_plain, N, K)).double()
+    ref, mag = da @ db.t(), da.abs() @ db.abs().t()
+    start = torch.randn(M, N, device="cuda")
+    bound = 2.0 * K * 2.0**-24 * mag + 1e-6
+    for dtype in (torch.float32, torch.bfloat16):
+        for accumulate in (False, True):
+            out = start.to(dtype)
+            want = ref * 0.5 + (out.double() if accumulate else 0.0)
+            mx.gemm(aq, asf, bq, bsf, out=out, accumulate=accumulate, alpha=0.5, bn=bn)
+            torch.cuda.synchronize()
+            native.check_status()
+            limit = bound + want.abs() * (2.0**-23 if dtype == torch.float32 else 2.0**-8)
+            assert ((out.double() - want).abs() <= limit).all(), f"{dtype} accumulate {accumulate}"
