@@ -8,6 +8,11 @@
 // TMEM columns: S [0,128) fp32, P [128,192) packed bf16, O [192,256) fp32. Two CTAs fit per SM, so
 // one CTA's softmax overlaps the other's tensor-core work.
 //
+// SPLIT (cached prefill and other padded batches, which keep 32-bit probabilities): P leaves the softmax as two bf16
+// numbers, its rounding and what the rounding left out (together 16 bits of mantissa and more), and O += P V runs once
+// for each. The low parts overwrite score columns that the same thread has read, so the low product is issued before
+// the next tile's scores and the high one after them: the tensor pipe stays ahead of the softmax, which is the bound.
+//
 // Documents never attend across their boundary: a tile's key range is clipped to its own document
 // and (with a window) to the last `window` positions. Sinks enter as sink_lse[h] = logsumexp of the
 // head's sink logits: the stored lse is logaddexp(lse, sink_lse) and the output is scaled to match.
@@ -106,6 +111,7 @@ __device__ __forceinline__ bool fwd_decode(const FlashFwdParams& p, int item, Fw
   return it.n_kv > 0;
 }
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(FA_THREADS, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const FlashFwdParams p) {
@@ -242,7 +248,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         ok = wait_all(p_full, gj & 1, KWU_ERR_TIMEOUT_MISC);
         if (!ok) break;
         tc_fence_after();
-        if (j + 1 < n_kv) issue_s(gj + 1, j + 2 == n_kv);
+        const uint64_t dV = make_smem_desc(smem_u32(sV + s * FA_TILE_BYTES), 8192, 1024, SWZ_128B);
+        uint32_t acc = j > 0 ? 1u : 0u;
+        if (!SPLIT && j + 1 < n_kv) issue_s(gj + 1, j + 2 == n_kv);
         ok = wait_all(&v_full[s], ph, KWU_ERR_TIMEOUT_FULL);
         if (!ok) break;
         if (j == 0) {
@@ -251,8 +259,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (!ok) break;
         }
         tc_fence_after();
-        const uint64_t dV = make_smem_desc(smem_u32(sV + s * FA_TILE_BYTES), 8192, 1024, SWZ_128B);
-        const uint32_t acc = j > 0 ? 1u : 0u;
+        if (SPLIT) {
+          // low parts: the first 32 of each thread's 64 score columns (keys 64 h .. 64 h + 63 at columns 64 h .. 64 h + 31)
+          if (leader) {
+#pragma unroll
+            for (int k = 0; k < FA_BN / 16; ++k)
+              mma_f16_ts(tO, tS + (k >> 2) * 64 + (k & 3) * 8, dV + 128 * k, idesc_o, k > 0 ? 1u : acc);
+          }
+          __syncwarp();
+          acc = 1u;
+          if (j + 1 < n_kv) issue_s(gj + 1, j + 2 == n_kv);   // in order behind the product that reads these columns
+        }
         if (leader) {
           mma_f16_ts(tO, tP, dV, idesc_o, acc);
 #pragma unroll
@@ -355,7 +372,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               }
               acc2[(e >> 1) & 1] = add_f32x2(acc2[(e >> 1) & 1], pack_f32x2(p0, p1));
               pk[c * 16 + e / 2] = pack_bf16(p0, p1);
+              if constexpr (SPLIT) {
+                const float2 hi = unpack_bf16(pk[c * 16 + e / 2]);
+                r[e / 2] = pack_bf16(p0 - hi.x, p1 - hi.y);
+              }
             }
+            if constexpr (SPLIT) tmem_st_x16(tS + lane_addr + col_base + c * 16, r);
           }
           unpack_f32x2(acc2[0], sum4[0], sum4[1]);
           unpack_f32x2(acc2[1], sum4[2], sum4[3]);
@@ -408,6 +430,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const float tot = fmaxf(lse, sl) + log1pf(__expf(-fabsf(lse - sl)));
           inv *= __expf(lse - tot);
           lse = tot;
+        }
+        if (SPLIT && !(l > 0.f && l < INFINITY)) {
+          // a row whose scores hold a NaN or an infinity, or are all -inf, has no probabilities: its output is zero
+          inv = 0.f;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = 0u;
         }
         if (qi < it.q_hi) {
           uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(qi) * p.Hq + h) * FA_D + half * 32);
@@ -487,6 +515,7 @@ KWU_API int kwu_attn_plan(const int* cu_seqlens, int ndocs, int tile, void* plan
   return 0;
 }
 
+template <bool SPLIT>
 static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
                           void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
                           int window, const float* sink_lse, float scale, void* q8, void* sf, void* stream,
@@ -504,7 +533,7 @@ static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, cons
   if ((rc = encode_tmap_2d(&tmV, v, ELEM_BF16, T, (uint64_t)Hkv * FA_D, v_ld, FA_BN, FA_D, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   static PerDeviceOnce attr;
   if (attr.pending()) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
     if (e != cudaSuccess) { set_last_error("flash_fwd attr: %s", cudaGetErrorString(e)); return 10; }
     attr.mark();
   }
@@ -524,7 +553,7 @@ static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, cons
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   long long items = static_cast<long long>(n_tiles) * Hq;
   int grid = static_cast<int>(items < 2LL * sms ? items : 2LL * sms);   // two resident CTAs per SM, each walks the item list
-  launch_k(flash_fwd_kernel, dim3(grid), dim3(FA_THREADS), FA_SMEM, reinterpret_cast<cudaStream_t>(stream), tmQ, tmK, tmV, p); kwu::count_launch();
+  launch_k(flash_fwd_kernel<SPLIT>, dim3(grid), dim3(FA_THREADS), FA_SMEM, reinterpret_cast<cudaStream_t>(stream), tmQ, tmK, tmV, p); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error("flash_fwd launch: %s", cudaGetErrorString(e)); return 11; }
   return 0;
@@ -533,7 +562,7 @@ static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, cons
 KWU_API int kwu_flash_fwd(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
                           void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
                           int window, const float* sink_lse, float scale, void* stream, int* status) {
-  return flash_fwd_impl(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
+  return flash_fwd_impl<false>(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
                         nullptr, nullptr, stream, status);
 }
 
@@ -544,6 +573,15 @@ KWU_API int kwu_flash_fwd_mx(const void* q, int q_ld, const void* k, int k_ld, c
                              void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
                              int window, const float* sink_lse, float scale, void* q8, void* sf, void* stream,
                              int* status) {
-  return flash_fwd_impl(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
+  return flash_fwd_impl<false>(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
                         q8, sf, stream, status);
+}
+
+// As kwu_flash_fwd with probabilities carried as a bf16 pair (SPLIT above): for callers that would otherwise form
+// attention in 32 bits.
+KWU_API int kwu_flash_fwd_split(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
+                                void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
+                                int window, const float* sink_lse, float scale, void* stream, int* status) {
+  return flash_fwd_impl<true>(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
+                              nullptr, nullptr, stream, status);
 }

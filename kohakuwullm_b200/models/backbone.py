@@ -123,6 +123,9 @@ class LMBackbone(nn.Module):
         if seq_info.packed and device.type == "cuda" and dtype == torch.bfloat16 and self.config.head_dim == 64 \
                 and attn_ops.native.available():
             plan = attn_ops.attention_plan(seq_info.cu_seqlens, seq_info.total_tokens)
+        elif not seq_info.packed and not torch.is_grad_enabled() and device.type == "cuda" and dtype == torch.bfloat16 \
+                and self.config.head_dim == 64:
+            plan = attn_ops.padded_plan(seq_info, device)
         return rope, plan
 
     def run_blocks(self, x, seq_info, rope, plan, cache=None, start: int = 0, end: int | None = None,

@@ -95,15 +95,25 @@ class Attention(nn.Module):
             out = varlen_attention(q, k, v, seq_info.cu_seqlens, seq_info.max_seqlen, window=self.window,
                                    sink_lse=self._sink_lse(), scale=self.scale, plan=plan)
             return self.o_proj(out.reshape(T, self.q_dim))
-        return self._forward_padded(x, seq_info, rope, cache, layer)
+        return self._forward_padded(x, seq_info, rope, cache, layer, plan)
 
-    def _forward_padded(self, x, seq_info, rope, cache, layer):
+    def _forward_padded(self, x, seq_info, rope, cache, layer, plan=None):
         B, S, _ = x.shape
         q, k, v = self._project(x.reshape(B * S, -1), rope)
         q = q.view(B, S, self.heads, self.head_dim)
         k = k.view(B, S, self.kv_heads, self.head_dim)
         v = v.view(B, S, self.kv_heads, self.head_dim)
         q_pos = seq_info.position_ids  # (B, S) absolute positions of the queries
+        # rows that count up from 0 over an empty cache (or without one) attend inside their own S columns only: packed
+        # documents of length S for the flash kernel
+        fused = plan is not None and seq_info.start is not None and (cache is None or seq_info.start == cache.length == 0) \
+            and getattr(self.attend, "__func__", None) is Attention.attend and not isinstance(self, SDPAAttention) \
+            and attn_ops.padded_supported(q, k, v, self.window)
+        if fused:
+            out = attn_ops.padded_attention(q, k, v, plan, self.window, self._sink_lse(), self.scale)
+            if cache is not None:
+                cache.append(layer, k, v, q_pos)
+            return self.o_proj(out.reshape(B, S, self.q_dim))
         if cache is not None:
             k, v, k_pos, k_valid = cache.append(layer, k, v, q_pos)
             if S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) \

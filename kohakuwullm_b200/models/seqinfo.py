@@ -8,9 +8,13 @@ Packed layout: ``tokens`` is (T,), ``cu_seqlens`` (N+1,) int32 marks document bo
 
 from __future__ import annotations
 
-from dataclasses import dataclass, replace
+from dataclasses import dataclass, field, replace
 
 import torch
+
+
+def _version(t: torch.Tensor) -> int:
+    return -1 if t.is_inference() else t._version
 
 
 @dataclass
@@ -21,6 +25,21 @@ class SeqInfo:
     num_seqs: int
     # host copy of the document lengths (kept so FLOP accounting and splitters never sync)
     lengths: tuple[int, ...] | None = None
+    # (first position, version of ``position_ids``) when every row is known to count up from one host-known position
+    _count: tuple[int, int] | None = field(default=None, init=False, repr=False, compare=False)
+
+    def __setattr__(self, name, value):
+        if name == "position_ids":
+            super().__setattr__("_count", None)
+        super().__setattr__(name, value)
+
+    @property
+    def start(self) -> int | None:
+        """Position of the first column when every row of a padded batch is ``start, start + 1, ...``, known without
+        reading the device; None when the positions were given, replaced or written to."""
+        if self._count is None or _version(self.position_ids) != self._count[1]:
+            return None
+        return self._count[0]
 
     @property
     def packed(self) -> bool:
@@ -59,11 +78,17 @@ class SeqInfo:
             pos = pos + offset.to(pos.device).reshape(-1, 1)
         elif offset:
             pos = pos + int(offset)
-        return cls(None, pos, seqlen, batch, None)
+        info = cls(None, pos, seqlen, batch, None)
+        if not isinstance(offset, torch.Tensor):
+            info._count = (int(offset), _version(pos))
+        return info
 
     def to(self, device, non_blocking: bool = False) -> "SeqInfo":
         cu = None if self.cu_seqlens is None else self.cu_seqlens.to(device, non_blocking=non_blocking)
-        return replace(self, cu_seqlens=cu, position_ids=self.position_ids.to(device, non_blocking=non_blocking))
+        new = replace(self, cu_seqlens=cu, position_ids=self.position_ids.to(device, non_blocking=non_blocking))
+        if self.start is not None:
+            new._count = (self.start, _version(new.position_ids))
+        return new
 
     def pin_memory(self) -> "SeqInfo":
         cu = None if self.cu_seqlens is None else self.cu_seqlens.pin_memory()

@@ -364,6 +364,45 @@ def attention_core(qkv, q_norm, k_norm, cos, sin, cu_seqlens, plan, sink_lse, Hq
                                 float(scale), float(eps), bool(do_norm), bool(emit_mx_grad), bool(emit_mx_out))
 
 
+# ------------------------------------------------------------------------------------ padded batches
+PADDED_MAX_TILES = 2048   # the plan kernel ranks the tiles against each other in one block
+
+
+def padded_plan(seq_info, device) -> torch.Tensor | None:
+    """Work lists (as :func:`attention_plan`) of a padded (B, S) batch whose rows count up from one position: B documents
+    of S tokens. None when the positions are not known to do that, a row is one token (the decode kernel's case), or the
+    lists would be too long."""
+    B, S = seq_info.position_ids.shape
+    if S < 2 or B < 1 or seq_info.start is None or B * ((S + 127) // 128) > PADDED_MAX_TILES or not native.available():
+        return None
+    return attention_plan(torch.arange(0, B * S + 1, S, dtype=torch.int32, device=device), B * S)
+
+
+def padded_supported(q, k, v, window) -> bool:
+    """q (B,S,H,64), k / v (B,S,Hkv,64) as the flash kernel reads them: token rows at one pitch, 16-byte aligned."""
+    return (not torch.is_grad_enabled() and q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16
+            and q.shape[-1] == 64 and q.shape[2] % k.shape[2] == 0 and (window is None or window > 0) and q.numel() > 0
+            and all(t.stride(3) == 1 and t.stride(2) == 64 and t.stride(0) == t.shape[1] * t.stride(1)
+                    and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+
+
+@torch.no_grad()
+def padded_attention(q, k, v, plan, window=None, sink_lse=None, scale=None):
+    """Causal attention of B rows of S tokens with probabilities that keep 16 and more mantissa bits (bf16 pairs): the
+    kernel form of ``Attention.attend`` for a prompt. q (B,S,H,64) -> (B,S,H,64)."""
+    L = native.require()
+    B, S, H, D = q.shape
+    out = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device)
+    lse = torch.empty(H, B * S, dtype=torch.float32, device=q.device)
+    rc = L.kwu_flash_fwd_split(
+        native.ptr(q), c_int(q.stride(1)), native.ptr(k), c_int(k.stride(1)), native.ptr(v), c_int(v.stride(1)),
+        native.ptr(out), native.ptr(lse), native.ptr(plan), c_int(plan.shape[0] // 2), c_int(B * S), c_int(H),
+        c_int(k.shape[2]), c_int(window or 0), native.ptr(sink_lse), c_float(scale if scale is not None else D ** -0.5),
+        native.stream_ptr(), native.ptr(native.status_word()))
+    native.check(rc, "flash_fwd_split")
+    return out
+
+
 # ------------------------------------------------------------------------------------ decode
 def decode_supported(q, k_cache) -> bool:
     return (native.available() and q.is_cuda and q.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16

@@ -324,3 +324,78 @@ def test_flash_forward_fp8_copy_of_output_equals_the_quantise_kernel():
     plain = attention_core(qkv, wq, wq, None, None, info.cu_seqlens, None, None, Hq, Hkv, None, 0.125, 1e-6, True)
     assert torch.equal(plain, out)
     native.check_status()
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,window,sinks", [
+    (1, 2, 4, 4, None, 0), (3, 41, 4, 2, 16, 2), (2, 127, 4, 1, None, 0), (2, 128, 8, 2, 1, 1), (1, 129, 4, 4, 128, 0),
+    (5, 257, 4, 2, 100, 4), (2, 1000, 6, 2, None, 1)])
+def test_padded_attention_is_as_exact_as_the_explicit_mask_form(B, S, H, Hkv, window, sinks):
+    """The kernel with bf16-pair probabilities against 64 bits, no further off than the fp32 explicit-mask form; both end in
+    a bf16 rounding (2^-9 of each value), which is nearly all of either error."""
+    from kohakuwullm_b200.models.components.attention import Attention
+    from kohakuwullm_b200.models.seqinfo import SeqInfo
+    from kohakuwullm_b200.ops import attention as A
+    from kohakuwullm_b200.ops import native
+
+    torch.manual_seed(S)
+    attn = Attention(64 * H, heads=H, kv_heads=Hkv, head_dim=64, window=window, sink=sinks > 0, num_sinks=max(sinks, 1)).cuda()
+    if sinks:
+        torch.nn.init.normal_(attn.sink, std=2.0)
+    qkv = torch.randn(B, S, H + 2 * Hkv, 64, device="cuda").bfloat16() * 2
+    q, k, v = qkv.split([H, Hkv, Hkv], 2)          # views at the pitch of the fused projection
+    info = SeqInfo.padded(B, S, device="cuda")
+    with torch.no_grad():
+        assert A.padded_supported(q, k, v, window)
+        out = A.padded_attention(q, k, v, A.padded_plan(info, q.device), window, attn._sink_lse(), attn.scale)
+        pos = info.position_ids
+        explicit = attn.attend(q, k, v, pos, pos, torch.ones(B, S, dtype=torch.bool, device="cuda"))
+        native.check_status()
+        s = torch.einsum("bshd,blhd->bhsl", q.double(), k.double().repeat_interleave(H // Hkv, 2)) * attn.scale
+        i = torch.arange(S, device="cuda")
+        ok = i[None, :] <= i[:, None]
+        if window:
+            ok &= i[:, None] - i[None, :] < window
+        lse = s.masked_fill(~ok, float("-inf")).logsumexp(-1)
+        if sinks:
+            lse = torch.logaddexp(lse, torch.logsumexp(attn.sink.double(), -1)[None, :, None])
+        p = torch.where(ok, torch.exp(s - lse[..., None]), 0.0)
+        want = torch.einsum("bhsl,blhd->bshd", p, v.double().repeat_interleave(H // Hkv, 2))
+    err, base = ((t.double() - want).norm() / want.norm() for t in (out, explicit))
+    assert err <= 1.02 * base and base < 2.0**-8, f"{err} against {base}"
+
+
+def test_padded_attention_route_and_degenerate_rows():
+    """Which calls take the kernel, and rows whose scores overflow: zero from both forms."""
+    from kohakuwullm_b200.models.components.attention import Attention
+    from kohakuwullm_b200.models.seqinfo import SeqInfo
+    from kohakuwullm_b200.ops import attention as A
+
+    B, S, H = 2, 70, 2
+    info = SeqInfo.padded(B, S, device="cuda")
+    assert info.start == 0 and SeqInfo.padded(B, S, offset=7).start == 7 and info.to("cpu").start == 0
+    given = SeqInfo.padded(B, S, device="cuda", offset=torch.tensor([0, 3]))
+    assert given.start is None and A.padded_plan(given, "cuda") is None
+    moved = SeqInfo.padded(1, S, offset=2)
+    moved.position_ids.add_(1)
+    assert moved.start is None
+    info.position_ids = info.position_ids + 1
+    assert info.start is None
+    q, k, v = (torch.randn(B, S, H, 64, device="cuda").bfloat16() for _ in range(3))
+    k[0, 5] = 3e38
+    q[0, 30] = 3e38                    # the score of key 5 and query 30 is +inf
+    q[1, 40] = float("nan")
+    attn = Attention(64 * H, heads=H, kv_heads=H, head_dim=64).cuda()
+    with torch.no_grad():
+        info = SeqInfo.padded(B, S, device="cuda")
+        pos = info.position_ids
+        want = attn.attend(q, k, v, pos, pos, torch.ones(B, S, dtype=torch.bool, device="cuda"))
+        out = A.padded_attention(q, k, v, A.padded_plan(info, q.device), None, None, attn.scale)
+    assert (want[0, 30] == 0).all() and (want[1, 40] == 0).all()
+    assert (out[0, 30] == 0).all() and (out[1, 40] == 0).all()
+    rest = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    rest[0] = False                    # scores against key 5 are huge in row 0: compared where they are ordinary
+    rest[1, 40] = False
+    torch.testing.assert_close(out[rest].float(), want[rest].float(), rtol=2.0**-7, atol=2.0**-9)
+    assert not A.padded_supported(q, k, v, 0)
+    with torch.enable_grad():
+        assert not A.padded_supported(q, k, v, None)
