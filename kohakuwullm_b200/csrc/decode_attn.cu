@@ -35,7 +35,9 @@ struct DecodeParams {
   long long v_sb, v_sl, v_sh;
   int B, H, Hkv, group;
   int kv_len, lo;                   // keys [lo, kv_len)
-  int n_chunks;
+  int n_chunks;                     // chunks the scratch has room for; the grid's width
+  const int* position;              // device position of the query: kv_len and lo follow from it (a captured step)
+  int window;
   float scale_log2e;
   float* part;                      // [B][H][n_chunks][66]: m, l, acc[64]
 };
@@ -50,14 +52,20 @@ decode_chunk_kernel(const DecodeParams p) {
   const int chunk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.group;
+  int kv_len = p.kv_len, lo = p.lo;
+  if (p.position) {
+    kv_len = min(*p.position + 1, p.kv_len);        // never past the cache
+    lo = (p.window > 0 && kv_len > p.window) ? kv_len - p.window : 0;
+    if (lo + chunk * DEC_CHUNK >= kv_len) return;   // the grid covers the longest context
+  }
   for (int i = tid; i < G * DEC_D; i += DEC_CHUNK) {
     const int g = i / DEC_D, d = i % DEC_D;
     s_q[g][d] = __bfloat162float(p.q[b * p.q_sb + (hk * G + g) * p.q_sh + d]) * p.scale_log2e;
   }
   __syncthreads();
   // phase 1: scores (log2 domain)
-  const int key = p.lo + chunk * DEC_CHUNK + tid;
-  const bool valid = key < p.kv_len;
+  const int key = lo + chunk * DEC_CHUNK + tid;
+  const bool valid = key < kv_len;
   float s[DEC_MAX_GROUP];
 #pragma unroll
   for (int g = 0; g < DEC_MAX_GROUP; ++g) s[g] = 0.f;
@@ -111,9 +119,9 @@ decode_chunk_kernel(const DecodeParams p) {
   float acc[DEC_MAX_GROUP][2];
 #pragma unroll
   for (int g = 0; g < DEC_MAX_GROUP; ++g) acc[g][0] = acc[g][1] = 0.f;
-  const int n_here = min(DEC_CHUNK, p.kv_len - (p.lo + chunk * DEC_CHUNK));
+  const int n_here = min(DEC_CHUNK, kv_len - (lo + chunk * DEC_CHUNK));
   for (int j = warp; j < n_here; j += 8) {
-    const long long pos = p.lo + chunk * DEC_CHUNK + j;
+    const long long pos = lo + chunk * DEC_CHUNK + j;
     const uint32_t vv = *reinterpret_cast<const uint32_t*>(p.v + b * p.v_sb + pos * p.v_sl + hk * p.v_sh + 2 * lane);
     const float2 f = unpack_bf16(vv);
 #pragma unroll
@@ -149,13 +157,19 @@ decode_chunk_kernel(const DecodeParams p) {
 
 // One block of 64 threads per (batch, head): merge the chunks.
 __global__ void __launch_bounds__(64)
-decode_combine_kernel(const float* __restrict__ part, int n_chunks, const float* __restrict__ sink, int n_sinks,
+decode_combine_kernel(const float* __restrict__ part, int max_chunks, const float* __restrict__ sink, int n_sinks,
                       __nv_bfloat16* __restrict__ out, long long o_sb, long long o_sh, float* __restrict__ lse,
-                      int H) {
+                      int H, const int* __restrict__ position, int window) {
+  int n_chunks = max_chunks;
+  if (position) {
+    int keys = *position + 1;
+    if (window > 0 && keys > window) keys = window;
+    n_chunks = min(max_chunks, (keys + DEC_CHUNK - 1) / DEC_CHUNK);
+  }
   const int bh = blockIdx.x;
   const int b = bh / H, h = bh % H;
   const int d = threadIdx.x;
-  const float* base = part + static_cast<size_t>(bh) * n_chunks * 66;
+  const float* base = part + static_cast<size_t>(bh) * max_chunks * 66;
   float m = -INFINITY;
   for (int c = 0; c < n_chunks; ++c) m = fmaxf(m, base[c * 66]);
   float l = 0.f, acc = 0.f;
@@ -192,12 +206,14 @@ KWU_API long long kwu_decode_scratch_floats(int B, int H, int max_keys) {
   return static_cast<long long>(B) * H * (chunks > 0 ? chunks : 1) * 66;
 }
 
-// Strides are in elements. window <= 0: all keys [0, kv_len). sink: (H, n_sinks) fp32 logits or null.
+// Strides are in elements. window <= 0: all keys [0, kv_len). sink: (H, n_sinks) fp32 logits or null. With `position`
+// (one int in device memory: the query's place in the cache) kv_len is the cache's capacity and the keys that exist are
+// found on the device, so that one captured launch serves every step.
 KWU_API int kwu_decode_attention(const void* q, long long q_sb, long long q_sh, const void* k, long long k_sb,
                                  long long k_sl, long long k_sh, const void* v, long long v_sb, long long v_sl,
                                  long long v_sh, void* out, long long o_sb, long long o_sh, float* lse, float* scratch,
                                  int B, int H, int Hkv, int kv_len, int window, float scale, const float* sink,
-                                 int n_sinks, void* stream) {
+                                 int n_sinks, const int* position, void* stream) {
   if (Hkv <= 0 || H % Hkv || H / Hkv > DEC_MAX_GROUP) { set_last_error("decode_attention: need H %% Hkv == 0 and group <= 8"); return 7; }
   if (kv_len <= 0 || B <= 0) { set_last_error("decode_attention: empty cache"); return 7; }
   if ((k_sl % 8) || (k_sh % 8) || (k_sb % 8) || (v_sl % 2) || (v_sh % 2)) { set_last_error("decode_attention: cache rows must be 16-byte aligned"); return 7; }
@@ -207,12 +223,15 @@ KWU_API int kwu_decode_attention(const void* q, long long q_sb, long long q_sh, 
   p.B = B; p.H = H; p.Hkv = Hkv; p.group = H / Hkv;
   p.kv_len = kv_len;
   p.lo = (window > 0 && kv_len > window) ? kv_len - window : 0;
+  p.position = position;
+  p.window = window;
   p.n_chunks = (kv_len - p.lo + DEC_CHUNK - 1) / DEC_CHUNK;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.part = scratch;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   decode_chunk_kernel<<<dim3(p.n_chunks, Hkv, B), DEC_CHUNK, 0, st>>>(p); kwu::count_launch();
-  decode_combine_kernel<<<B * H, 64, 0, st>>>(scratch, p.n_chunks, sink, n_sinks, (__nv_bfloat16*)out, o_sb, o_sh, lse, H); kwu::count_launch();
+  decode_combine_kernel<<<B * H, 64, 0, st>>>(scratch, p.n_chunks, sink, n_sinks, (__nv_bfloat16*)out, o_sb, o_sh, lse, H,
+                                                 position, window); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error("decode_attention launch: %s", cudaGetErrorString(e)); return 11; }
   return 0;

@@ -85,6 +85,87 @@ def advance(tokens: torch.Tensor, nxt: torch.Tensor, finished: torch.Tensor, sto
     return torch.cat([tokens, nxt[:, None]], dim=1), finished | hit
 
 
+class StepGraph:
+    """One cached decode step (embedding to logits of one new token a row) captured as a CUDA graph.
+
+    A step is 15 to 20 short kernels a layer; issued from Python they leave the GPU idle for most of the step, replayed
+    they follow each other. The position lives on the device (``KVCache.hold_position``), so one capture serves every
+    remaining token of the call. ``earlier``: a finished capture whose memory this one takes over."""
+
+    MIN_STEPS = 3     # a capture costs about a step issued from Python, so it pays from the third on
+
+    def __init__(self, backbone, cache, token: torch.Tensor, earlier: "StepGraph | None" = None):
+        self.token = token.clone()
+        self.graph = torch.cuda.CUDAGraph()
+        length = cache.length
+        cache.hold_position(token.device)
+        stream = torch.cuda.Stream(device=token.device)
+        stream.wait_stream(torch.cuda.current_stream(token.device))
+        try:
+            with torch.cuda.stream(stream):
+                # thread-local: other threads of the program may go on allocating and synchronising
+                pool = () if earlier is None else (earlier.graph.pool(),)
+                self.graph.capture_begin(*pool, capture_error_mode="thread_local")
+                try:
+                    hidden = backbone(self.token, cache.seq_info(self.token), cache=cache)
+                    self.logits = backbone.head.logits(hidden[:, -1])
+                finally:
+                    self.graph.capture_end()
+        except BaseException:
+            cache.position = None
+            raise
+        finally:
+            cache.length, cache._pending = length, 0      # nothing has run yet
+
+    def __call__(self, cache, token: torch.Tensor) -> torch.Tensor:
+        if cache.length + 1 > cache.max_len:
+            raise RuntimeError(f"KV cache overflow: {cache.length + 1} > max_len {cache.max_len}")
+        self.token.copy_(token)
+        self.graph.replay()
+        cache.length += 1
+        return self.logits
+
+
+def capturable(backbone, tokens: torch.Tensor) -> bool:
+    """Whether a cached one-token step of this model is a fixed sequence of kernels: every module is one whose decode path
+    reads nothing back to the host, runs on the native kernels, and carries no hooks or replaced methods that a replay
+    would skip."""
+    from torch.nn.modules import module as hooks
+
+    from kohakuwullm_b200.models.backbone import LMBackbone
+    from kohakuwullm_b200.models.block import DecoderBlock
+    from kohakuwullm_b200.models.components import attention, mlp, moe, norm, posenc
+    from kohakuwullm_b200.models.head import LMHead
+    from kohakuwullm_b200.ops import native
+
+    plain = (LMBackbone, DecoderBlock, LMHead, mlp.Linear, mlp.GLUMLP, mlp.GeGLUMLP, mlp.GELUMLP, norm.RMSNorm,
+             norm.GemmaRMSNorm, norm.LayerNorm, norm.DyT, posenc.RoPE, posenc.NoPE, torch.nn.Embedding, torch.nn.ModuleList,
+             torch.nn.Identity)
+    if type(backbone) is not LMBackbone or not tokens.is_cuda or not native.available() \
+            or torch.cuda.is_current_stream_capturing() or hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
+        return False
+    if backbone.embed.weight.dtype != torch.bfloat16 or backbone.config.head_dim != 64:
+        return False
+    if any(t.device != tokens.device for group in (backbone.parameters(), backbone.buffers()) for t in group):
+        return False
+    for m in backbone.modules():
+        if m._forward_hooks or m._forward_pre_hooks or any(callable(v) for v in vars(m).values()):
+            return False
+        if type(m) is attention.Attention:
+            if m.heads % m.kv_heads or m.heads // m.kv_heads > 8 or \
+                    not (m.qk_norm or type(backbone.pos_enc) is posenc.RoPE):     # q would be a view of the projection
+                return False
+        elif type(m) is moe.MoEMLP:
+            w = m.router.weight
+            if m.ep_world > 1 or m.expert_path not in (None, "grouped") or type(m.router) is not moe.TopKRouter \
+                    or m.router.num_groups > 1 or w.shape[0] > 128 or w.shape[0] % 8 or w.dtype != torch.float32 \
+                    or m.w_in.dtype != torch.bfloat16 or m.dim % 64 or m.w_in.shape[1] % 128:
+                return False
+        elif type(m) is not moe.TopKRouter and type(m) not in plain:
+            return False
+    return True
+
+
 class LocalGenerator:
     def __init__(self, backbone, eos_id: int = 0, stop_ids: Sequence[int] = (), use_cache: bool = True,
                  static_cache: bool = True):
@@ -92,6 +173,7 @@ class LocalGenerator:
         self.stop_ids = tuple(stop_ids) or (eos_id,)
         self.use_cache, self.static_cache = use_cache, static_cache
         self._rng: dict[str, torch.Generator] = {}
+        self._captures: dict[str, StepGraph] = {}     # the last finished capture of a device, for its memory
 
     def rng(self, device) -> torch.Generator:
         key = str(device)
@@ -113,17 +195,29 @@ class LocalGenerator:
         gen = self.rng(prompt.device)
         cache = KVCache.from_config(bb.config, S + max_new_tokens, static=self.static_cache) if self.use_cache else None
         step_in = prompt
-        for _ in range(max_new_tokens):
-            if cache is not None:
-                hidden = bb(step_in, cache.seq_info(step_in), cache=cache)
+        graph, graphs = None, cache is not None and self.static_cache and capturable(bb, prompt)
+        for i in range(max_new_tokens):
+            # the first one-token step is issued directly: it loads kernels and builds what later ones find
+            if graphs and graph is None and i >= 2 and max_new_tokens - i >= StepGraph.MIN_STEPS:
+                try:
+                    graph = StepGraph(bb, cache, step_in, self._captures.pop(str(prompt.device), None))
+                except RuntimeError:       # what cannot be captured is issued directly, and raises there if it is wrong
+                    graphs = False
+            if graph is not None:
+                logits = graph(cache, step_in)
             else:
-                hidden = bb(tokens, SeqInfo.padded(rows, tokens.shape[1], device=tokens.device))
-            logits = bb.head.logits(hidden[:, -1])
+                if cache is not None:
+                    hidden = bb(step_in, cache.seq_info(step_in), cache=cache)
+                else:
+                    hidden = bb(tokens, SeqInfo.padded(rows, tokens.shape[1], device=tokens.device))
+                logits = bb.head.logits(hidden[:, -1])
             nxt = sample(logits, generator=gen, **sampling)
             tokens, finished = advance(tokens, nxt, finished, self.stop_ids, self.eos)
             step_in = tokens[:, -1:]
             if bool(finished.all()):
                 break
+        if graph is not None:
+            self._captures[str(prompt.device)] = graph
         bb.train(was_training)
         return tokens
 

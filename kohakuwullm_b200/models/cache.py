@@ -21,6 +21,9 @@ class KVCache:
         self.v: list[torch.Tensor | None] = [None] * num_layers
         self.length = 0
         self._pending = 0
+        # while one-token steps are captured: the next position as device integers (int64 for indexing, int32 for the
+        # decode kernel), advanced by the step itself
+        self.position: tuple[torch.Tensor, torch.Tensor] | None = None
 
     @classmethod
     def from_config(cls, config, max_len: int, static: bool = True, num_layers: int | None = None):
@@ -29,6 +32,8 @@ class KVCache:
     def seq_info(self, tokens: torch.Tensor) -> SeqInfo:
         """Layout of the next ``tokens`` (B,S): positions continue after the cached prefix."""
         b, s = tokens.shape
+        if self.position is not None:
+            return SeqInfo(None, self.position[0].view(1, 1).expand(b, s), s, b, None)
         return SeqInfo.padded(b, s, device=tokens.device, offset=self.length)
 
     def append(self, layer: int, k: torch.Tensor, v: torch.Tensor, q_pos: torch.Tensor):
@@ -41,6 +46,11 @@ class KVCache:
             shape = (B, self.max_len, *k.shape[2:])
             self.k[layer] = torch.zeros(shape, dtype=k.dtype, device=k.device)
             self.v[layer] = torch.zeros(shape, dtype=v.dtype, device=v.device)
+        if self.position is not None:
+            self.k[layer].index_copy_(1, self.position[0], k)
+            self.v[layer].index_copy_(1, self.position[0], v)
+            self._pending = S
+            return self.k[layer], self.v[layer], None, None
         self.k[layer][:, self.length:end] = k
         self.v[layer][:, self.length:end] = v
         self._pending = S
@@ -49,7 +59,16 @@ class KVCache:
         valid = pos < end
         return self.k[layer][:, :used], self.v[layer][:, :used], pos, valid
 
+    def hold_position(self, device) -> None:
+        """One-token steps from here on read their position from the device (every buffer exists: a static cache past
+        its first step), so that a captured step can be replayed for each next token."""
+        self.position = (torch.full((1,), self.length, dtype=torch.int64, device=device),
+                         torch.full((1,), self.length, dtype=torch.int32, device=device))
+
     def advance(self) -> None:
+        if self.position is not None:
+            for p in self.position:
+                p += self._pending
         self.length += self._pending
         self._pending = 0
 

@@ -119,7 +119,9 @@ class Attention(nn.Module):
             if S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) \
                     and q.is_contiguous():
                 # one new token per row: split-KV decode kernel straight over the cache buffers
-                out = attn_ops.decode_attention(q[:, 0], k, v, cache.length + 1, self.window, self.scale, self.sink)
+                held = cache.position is not None
+                out = attn_ops.decode_attention(q[:, 0], k, v, k.shape[1] if held else cache.length + 1, self.window,
+                                                self.scale, self.sink, position=cache.position[1] if held else None)
                 return self.o_proj(out.reshape(B, 1, self.q_dim))
         else:
             k_pos = q_pos

@@ -409,15 +409,13 @@ def decode_supported(q, k_cache) -> bool:
             and q.shape[-1] == 64 and q.shape[-2] % k_cache.shape[-2] == 0 and q.shape[-2] // k_cache.shape[-2] <= 8)
 
 
-_decode_scratch: dict = {}
-
-
 @torch.no_grad()
 def decode_attention(q, k_cache, v_cache, kv_len: int, window: int | None = None, scale: float | None = None,
-                     sink: torch.Tensor | None = None, return_lse: bool = False):
+                     sink: torch.Tensor | None = None, return_lse: bool = False, position: torch.Tensor | None = None):
     """One new token per row against a KV cache: q (B,H,64); caches (B,L_max,Hkv,64); the query sits at
     position ``kv_len - 1`` and attends keys ``[max(0, kv_len - window), kv_len)``. ``sink`` (H,S) fp32 learned
-    sink logits join the softmax denominator. Split-KV kernel in ``csrc/decode_attn.cu``."""
+    sink logits join the softmax denominator. With ``position`` (one int32 on the device) the query sits there instead and
+    ``kv_len`` is only an upper bound. Split-KV kernel in ``csrc/decode_attn.cu``."""
     L = native.require()
     B, H, D = q.shape
     Hkv = k_cache.shape[2]
@@ -425,10 +423,7 @@ def decode_attention(q, k_cache, v_cache, kv_len: int, window: int | None = None
     out = torch.empty(B, H, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, H, dtype=torch.float32, device=q.device)
     need = int(L.kwu_decode_scratch_floats(ctypes.c_int(B), ctypes.c_int(H), ctypes.c_int(k_cache.shape[1])))
-    key = (q.device, need)
-    scratch = _decode_scratch.get(key)
-    if scratch is None:
-        scratch = _decode_scratch[key] = torch.empty(need, dtype=torch.float32, device=q.device)
+    scratch = torch.empty(need, dtype=torch.float32, device=q.device)
     sink_f = sink.detach().float().contiguous() if sink is not None else None
     ll = ctypes.c_longlong
     rc = L.kwu_decode_attention(
@@ -438,7 +433,7 @@ def decode_attention(q, k_cache, v_cache, kv_len: int, window: int | None = None
         native.ptr(out), ll(out.stride(0)), ll(out.stride(1)), native.ptr(lse), native.ptr(scratch),
         ctypes.c_int(B), ctypes.c_int(H), ctypes.c_int(Hkv), ctypes.c_int(int(kv_len)), ctypes.c_int(int(window or 0)),
         ctypes.c_float(scale), native.ptr(sink_f), ctypes.c_int(0 if sink_f is None else sink_f.shape[1]),
-        native.stream_ptr())
+        native.ptr(position), native.stream_ptr())
     native.check(rc, "decode_attention")
     return (out, lse) if return_lse else out
 
