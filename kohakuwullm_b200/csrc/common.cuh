@@ -97,6 +97,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// One arrival for the whole warp (the barrier counts warps): arrivals of 32 lanes on one barrier are served one by one.
+// What the lanes did before is ordered before the arrival by the warp barrier.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
 // One probe of the barrier. A thread whose phase is not complete yet is suspended by the hardware until the
 // phase completes or `KWU_WAIT_SUSPEND_NS` have passed, whichever is first, so a waiting warp costs no issue
 // slots and no ALU cycles while it waits (a busy loop of probes took a large share of both from the warps

@@ -150,11 +150,11 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
       mbar_init(&qd_empty[s], 1);
     }
     mbar_init(sdp_full, 1);
-    mbar_init(p_ready, 256);
+    mbar_init(p_ready, 8);
     mbar_init(dp_full, 1);
-    mbar_init(ds_ready, 256);
+    mbar_init(ds_ready, 8);
     mbar_init(acc_done, 1);
-    mbar_init(acc_free, 256);
+    mbar_init(acc_free, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -401,7 +401,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
           tmem_st_x16(tS + lane_addr + c * 32, pp);
           tmem_st_wait();
           tc_fence_before();
-          mbar_arrive(p_ready);
+          mbar_arrive_warp(p_ready);
           // phase 2: dS^T = P^T o (dP^T * scale - delta)
           bool fine = mbar_wait(dp_full, gi & 1, abort_flag, p.status, KWU_ERR_TIMEOUT_ACC_FULL);
           fine = __all_sync(0xffffffffu, fine);
@@ -426,7 +426,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
           tmem_st_x16(tDP + lane_addr + c * 32, dd);
           tmem_st_wait();
           tc_fence_before();
-          mbar_arrive(ds_ready);
+          mbar_arrive_warp(ds_ready);
           return true;
         };
         ok = need_mask ? tile(BoolC<true>{}) : tile(BoolC<false>{});
@@ -446,7 +446,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
         tmem_ld_x32(src + 32, o + 32);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(acc_free);   // the next item's first products may overwrite the accumulators now
+        mbar_arrive_warp(acc_free);   // the next item's first products may overwrite the accumulators now
         if (kj < de) {
           if (p.dk_part) {
             float4* dst = reinterpret_cast<float4*>((which == 0 ? p.dv_part : p.dk_part) +
@@ -548,11 +548,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
     }
     mbar_init(&sdp_full[0], 1);
     mbar_init(&sdp_full[1], 1);
-    mbar_init(p_ready, 256);
+    mbar_init(p_ready, 8);
     mbar_init(dp_full, 1);
     mbar_init(acc_done, 1);
     mbar_init(q_empty, 1);
-    mbar_init(acc_free, 256);
+    mbar_init(acc_free, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -737,7 +737,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
           tmem_st_x16(tSj + lane_addr + c * 32, dd);
           tmem_st_wait();
           tc_fence_before();
-          mbar_arrive(p_ready);
+          mbar_arrive_warp(p_ready);
           return true;
         };
         ok = need_mask ? tile(BoolC<true>{}) : tile(BoolC<false>{});
@@ -753,7 +753,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
       tmem_ld_x32(tDQ + lane_addr + half * 32, o);
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(acc_free);
+      mbar_arrive_warp(acc_free);
       if (qi < q_hi) {
         uint4* dst = reinterpret_cast<uint4*>(p.dq + (static_cast<size_t>(qi) * p.Hq + h) * FB_D + half * 32);
 #pragma unroll

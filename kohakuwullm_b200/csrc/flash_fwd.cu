@@ -150,10 +150,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&v_empty[s], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(p_full, 256);
+    mbar_init(p_full, 8);
     mbar_init(o_done, 1);
     mbar_init(q_empty, 1);
-    mbar_init(o_free, 256);
+    mbar_init(o_free, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -291,6 +291,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int row = quarter * 32 + lane;     // query row inside the tile == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t col_base = half * 64;
+    // the two warps that share a row meet on a named barrier of their own
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory"); };
     int g = 0;
     bool ok = true;
     for (int rnd = 0; rnd * static_cast<int>(gridDim.x) < n_items; ++rnd) {
@@ -339,7 +341,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // exchange with the thread that owns the other half of the row (buffers alternate per tile)
         float* xbuf = s_rowmax + (gj & 1) * 256;
         xbuf[half * 128 + row] = mx;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        pair_sync();
         mx = fmaxf(fmaxf(mx, xbuf[(half ^ 1) * 128 + row]), m);
         if (!ok) continue;
         const float alpha = fast_exp2((m - mx) * p.scale_log2);
@@ -404,7 +406,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tmem_st_x32(tP + lane_addr + half * 32, pk);
         tmem_st_wait();
         tc_fence_before();
-        mbar_arrive(p_full);
+        mbar_arrive_warp(p_full);
       }
       // ---------------------------------------------------------------- epilogue of the item
       if (ok) {
@@ -414,7 +416,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // total row sum = own partial + the partner's (both are relative to the same final maximum)
       float* lbuf = s_rowmax + 512;
       lbuf[half * 128 + row] = l;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      pair_sync();
       l += lbuf[(half ^ 1) * 128 + row];
       if (ok) {
         tc_fence_after();
@@ -422,7 +424,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tmem_ld_x32(tO + lane_addr + half * 32, o);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(o_free);   // the next item's first product may overwrite O now
+        mbar_arrive_warp(o_free);   // the next item's first product may overwrite O now
         float lse = (m * p.scale_log2 + log2f(l)) * 0.6931471805599453f;  // natural log
         float inv = 1.f / l;
         if (p.sink_lse) {
