@@ -538,6 +538,88 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ------------------------------------------------------------------ products of a few rows
+// C[m, n] = alpha * sum_k A[m, k] B[n, k] for M <= 16, both K-major: the step of a decode. It is a stream of B through the
+// chip once; a 128-row tile spends its time on the serial k-blocks of a few CTAs instead. Mean of the products of a decode
+// step, tile / this, us: 17 layers of 768 wide and the 65536-wide head, one row 8.8 / 4.1; 22 layers of 1280, eight rows
+// 12.4 / 6.1. The head alone (2 x 65536 x 1280) takes 37.6 us, 4.5 TB/s.
+// A CTA owns 16 rows of B, its eight warps a slice of the contraction each. B's rows are the M side of
+// mma.m16n8k16 and A's rows (up to 8 per product) the N side. A lane loads 16 bytes of rows g and g + 8 of B and of row g
+// of A at the same eight k's; the products take them as four pairs, so the order of k inside a 32-wide step is permuted
+// alike on both sides. Up to four steps of loads are in flight per lane. The eight partial sums meet in shared memory in
+// a fixed order.
+constexpr int FEW_WARPS = 8, FEW_UNROLL = 4;
+
+__device__ __forceinline__ void mma_m16n8k16_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                  uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int HALVES>   // 8 rows of A each
+__global__ void __launch_bounds__(FEW_WARPS * 32)
+gemm_few_rows_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, void* __restrict__ C, int M,
+                     int N, int K, int lda, int ldb, int ldc, int out_fp32, float alpha) {
+  pdl_sync();   // nothing of the previous kernel is read above this line
+  __shared__ float s_part[FEW_WARPS][HALVES * 8][17];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * 16;
+  const int steps = (K + 31) / 32;
+  const int s_begin = steps * warp / FEW_WARPS, s_end = steps * (warp + 1) / FEW_WARPS;
+  const __nv_bfloat16* b0 = B + static_cast<size_t>(n0 + g) * ldb + 8 * t;
+  const __nv_bfloat16* b1 = b0 + static_cast<size_t>(8) * ldb;
+  const bool n_lo = n0 + g < N, n_hi = n0 + g + 8 < N;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  float acc[HALVES][4];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[h][i] = 0.f;
+  for (int s = s_begin; s < s_end; s += FEW_UNROLL) {
+    uint4 w0[FEW_UNROLL], w1[FEW_UNROLL], x[FEW_UNROLL][HALVES];
+#pragma unroll
+    for (int u = 0; u < FEW_UNROLL; ++u) {
+      const int k = (s + u) * 32;
+      const bool in = s + u < s_end && k + 8 * t < K;     // K is a multiple of 8
+      w0[u] = in && n_lo ? __ldg(reinterpret_cast<const uint4*>(b0 + k)) : zero;
+      w1[u] = in && n_hi ? __ldg(reinterpret_cast<const uint4*>(b1 + k)) : zero;
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        const int m = 8 * h + g;
+        x[u][h] = in && m < M ? __ldg(reinterpret_cast<const uint4*>(A + static_cast<size_t>(m) * lda + k + 8 * t)) : zero;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < FEW_UNROLL; ++u)
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        mma_m16n8k16_bf16(acc[h], w0[u].x, w1[u].x, w0[u].y, w1[u].y, x[u][h].x, x[u][h].y);
+        mma_m16n8k16_bf16(acc[h], w0[u].z, w1[u].z, w0[u].w, w1[u].w, x[u][h].z, x[u][h].w);
+      }
+  }
+  // acc: rows g, g + 8 of B by rows 2 t, 2 t + 1 of A
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h) {
+    s_part[warp][8 * h + 2 * t][g] = acc[h][0];
+    s_part[warp][8 * h + 2 * t + 1][g] = acc[h][1];
+    s_part[warp][8 * h + 2 * t][g + 8] = acc[h][2];
+    s_part[warp][8 * h + 2 * t + 1][g + 8] = acc[h][3];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < HALVES * 128; i += FEW_WARPS * 32) {
+    const int m = i >> 4, n = i & 15;
+    if (m >= M || n0 + n >= N) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < FEW_WARPS; ++w) v += s_part[w][m][n];
+    v *= alpha;
+    const size_t at = static_cast<size_t>(m) * ldc + n0 + n;
+    if (out_fp32) reinterpret_cast<float*>(C)[at] = v;
+    else reinterpret_cast<__nv_bfloat16*>(C)[at] = __float2bfloat16(v);
+  }
+}
+
 // ------------------------------------------------------------------ host launcher
 static int num_sms() {
   static int n = 0;
@@ -717,6 +799,16 @@ KWU_API int kwu_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   using namespace kwu;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // up to 16 rows against a K-major B are a stream of B, which needs no tensor maps; 16-byte loads want aligned rows
+  if (bn == 0 && max_ctas == 0 && M <= 16 && !a_mn && !b_mn && !accumulate && K % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0 &&
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0) {
+    auto kern = M <= 8 ? gemm_few_rows_kernel<1> : gemm_few_rows_kernel<2>;
+    launch_k(kern, dim3((N + 15) / 16), dim3(FEW_WARPS * 32), 0, st, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, M, N, K,
+             lda, ldb, ldc, out_fp32, alpha); kwu::count_launch();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { set_last_error("gemm_few_rows launch: %s", cudaGetErrorString(e)); return 11; }
+    return 0;
+  }
   TilePick pick{bn > 1000 ? 2 : 1, bn > 1000 ? bn - 1000 : bn, 1};
   if (bn == 0) pick = pick_tile(M, N, K, b_mn != 0, out_fp32 && accumulate, 0, 2, max_ctas);
   if (pick.bn < 64 || pick.bn > 256 || pick.bn % 32) {

@@ -115,3 +115,26 @@ def test_cross_entropy_partials_fold(vocab):
     want_ce, want_lse = linear_cross_entropy_reference(h, w, labels)
     torch.testing.assert_close(lse, want_lse, rtol=1e-4, atol=1e-3)
     torch.testing.assert_close(ce, want_ce, rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K", [(16, 8), (40, 264), (768, 768), (1000, 2056), (65536, 128)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_few_rows_against_64_bits(M, N, K, out_dtype):
+    """Products of up to 16 rows (and 17, the first of the tiled kernel): cut rows of B, cut slices of the contraction,
+    operands and outputs that are views. An fp32 sum of K exact products is off by at most 2 K 2^-24 of the sum of
+    magnitudes, a bf16 result by another 2^-9 of itself."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.gemm import matmul
+
+    torch.manual_seed(M + N)
+    a = torch.randn(M, K + 8, device="cuda").bfloat16()[:, :K]
+    b = torch.randn(N, K + 16, device="cuda").bfloat16()[:, 8:K + 8]
+    store = torch.full((M, N + 3), 7.0, device="cuda", dtype=out_dtype)
+    out = matmul(a, b, out=store[:, :N], alpha=0.5)
+    torch.cuda.synchronize()
+    native.check_status()
+    want = 0.5 * a.double() @ b.double().t()
+    limit = K * 2.0**-24 * (a.double().abs() @ b.double().abs().t()) + want.abs() * (2.0**-8 if out_dtype == torch.bfloat16 else 2.0**-23) + 1e-7
+    assert ((out.double() - want).abs() <= limit).all()
+    assert (store[:, N:] == 7).all()
