@@ -38,6 +38,13 @@ class KVCache:
 
     def append(self, layer: int, k: torch.Tensor, v: torch.Tensor, q_pos: torch.Tensor):
         """Store this step's keys/values; returns ``(k_all, v_all, key_positions, key_valid)``."""
+        k_all, v_all = self.store(layer, k, v)
+        B, used = k_all.shape[:2]
+        pos = torch.arange(used, device=k.device)[None, :].expand(B, used)
+        return k_all, v_all, pos, pos < self.length + k.shape[1]
+
+    def store(self, layer: int, k: torch.Tensor, v: torch.Tensor):
+        """:meth:`append` for kernels that know which keys exist: returns ``(k_all, v_all)`` alone."""
         B, S = k.shape[:2]
         end = self.length + S
         if end > self.max_len:
@@ -50,14 +57,12 @@ class KVCache:
             self.k[layer].index_copy_(1, self.position[0], k)
             self.v[layer].index_copy_(1, self.position[0], v)
             self._pending = S
-            return self.k[layer], self.v[layer], None, None
+            return self.k[layer], self.v[layer]
         self.k[layer][:, self.length:end] = k
         self.v[layer][:, self.length:end] = v
         self._pending = S
         used = self.max_len if self.static else end
-        pos = torch.arange(used, device=k.device)[None, :].expand(B, used)
-        valid = pos < end
-        return self.k[layer][:, :used], self.v[layer][:, :used], pos, valid
+        return self.k[layer][:, :used], self.v[layer][:, :used]
 
     def hold_position(self, device) -> None:
         """One-token steps from here on read their position from the device (every buffer exists: a static cache past

@@ -112,12 +112,16 @@ class Attention(nn.Module):
         if fused:
             out = attn_ops.padded_attention(q, k, v, plan, self.window, self._sink_lse(), self.scale)
             if cache is not None:
-                cache.append(layer, k, v, q_pos)
+                cache.store(layer, k, v)
             return self.o_proj(out.reshape(B, S, self.q_dim))
         if cache is not None:
-            k, v, k_pos, k_valid = cache.append(layer, k, v, q_pos)
-            if S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) \
-                    and q.is_contiguous():
+            # the decode kernel needs no key positions
+            decode = S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) and q.is_contiguous()
+            if decode:
+                k, v = cache.store(layer, k, v)
+            else:
+                k, v, k_pos, k_valid = cache.append(layer, k, v, q_pos)
+            if decode:
                 # one new token per row: split-KV decode kernel straight over the cache buffers
                 held = cache.position is not None
                 out = attn_ops.decode_attention(q[:, 0], k, v, k.shape[1] if held else cache.length + 1, self.window,

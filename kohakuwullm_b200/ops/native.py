@@ -57,16 +57,24 @@ def lib() -> ctypes.CDLL:
     return handle
 
 
+# These run once or more per operator call, so they ask torch only what can change between two calls: an initialised
+# CUDA context answers "is there a device", and a device's capability is looked up once.
+_capable: dict[int, bool] = {}
+
+
 def available() -> bool:
     """True when the native kernels can run here (CUDA device of compute capability 10.x)."""
-    if not torch.cuda.is_available():
-        return False
-    major, _ = torch.cuda.get_device_capability()
-    return major == 10
+    if not torch.cuda.is_initialized():
+        return torch.cuda.is_available() and torch.cuda.get_device_capability()[0] == 10
+    dev = torch.cuda.current_device()
+    known = _capable.get(dev)
+    if known is None:
+        known = _capable[dev] = torch.cuda.get_device_capability(dev)[0] == 10
+    return known
 
 
 def require() -> ctypes.CDLL:
-    if not torch.cuda.is_available():
+    if not torch.cuda.is_initialized() and not torch.cuda.is_available():
         raise NativeError("native kernels need a CUDA device")
     return lib()
 
@@ -78,7 +86,7 @@ def check(rc: int, what: str) -> None:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
