@@ -74,12 +74,15 @@ struct GemmParams {
   //      a block of `group_b_rows` rows of B (K-major: output rows; MN-major: contraction rows)
   //   2: contraction grouped by expert (weight gradients): C[e] (+)= A[rows_e]^T B[rows_e] with
   //      rows_e = [group_offsets[e], group_offsets[e+1]); C advances by c_group_rows rows per expert
+  //   3: a batch of products of one size: matrix i owns rows [i, i + 1) * c_group_rows of A and C (whole tiles) and a
+  //      block of `group_b_rows` rows of B
   int group_mode;
   const int4* group_tiles;
   const int* group_offsets;
   int group_b_rows;
   int num_groups;
   int c_group_rows;
+  float diag;       // added on the diagonal of every matrix (mode 3): C = alpha * A B + diag * I
   // scatter epilogue (bf16 EPI_STORE only): output row r goes to the byte address row_ptrs[r] (0: row is
   // dropped) instead of C + r*ldc. The addresses may be peer-mapped memory of another GPU: the expert-
   // parallel combine / gradient return is then done by the GEMM's own epilogue stores, tile by tile.
@@ -127,6 +130,14 @@ __device__ __forceinline__ bool decode_tile(const GemmParams& p, int tile, int n
     t.nkb = (p.group_offsets[e + 1] - t.k_begin) / GEMM_BK;
     t.c_row_off = e * p.c_group_rows;
     return t.nkb > 0;
+  }
+  if (p.group_mode == 3) {
+    const int mt = p.c_group_rows / TM, per = mt * p.tiles_n;
+    const int i = tile / per, r = tile - i * per;
+    t.m0 = i * p.c_group_rows + (r % mt) * TM;
+    t.n0 = (r / mt) * p.bn;
+    t.b_row_off = i * p.group_b_rows;
+    return true;
   }
   if (p.group_mode == 1) {
     const int tm = tile / p.tiles_n;
@@ -415,6 +426,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]) * p.alpha;
+            if (p.diag != 0.f) {
+              const int d = row % p.c_group_rows - col0;
+              if (__any_sync(0xffffffffu, d >= 0 && d < 32)) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (j == d) f[j] += p.diag;
+              }
+            }
           }
           if (p.out_mode == OUT_TMA_BF16) {
             // 64-column boxes: 128-byte rows, 16-byte units XORed with the row (the TMA's 128-byte swizzle);
@@ -640,6 +659,7 @@ struct GroupArgs {
   int num_groups = 1;
   int c_rows = 0;
   int row_tiles = 0;  // mode 1: number of entries in `tiles`
+  float diag = 0.f;   // mode 3
   const long long* row_ptrs = nullptr;
 };
 
@@ -688,7 +708,7 @@ static int launch_gemm(int BN, const void* A, const void* B, void* C, int M, int
   p.tiles_n = (N + BN - 1) / BN;
   p.status = status;
   p.group_mode = ga.mode; p.group_tiles = ga.tiles; p.group_offsets = ga.offsets;
-  p.group_b_rows = ga.b_rows; p.num_groups = ga.num_groups; p.c_group_rows = ga.c_rows;
+  p.group_b_rows = ga.b_rows; p.num_groups = ga.num_groups; p.c_group_rows = ga.c_rows; p.diag = ga.diag;
   p.row_ptrs = (EPI == EPI_STORE && !out_fp32) ? ga.row_ptrs : nullptr;
   p.labels = ea.labels; p.partial = ea.partial; p.target_logit = ea.target_logit;
   p.lse = ea.lse; p.coef_p = ea.coef_p; p.coef_y = ea.coef_y;
@@ -944,6 +964,35 @@ KWU_API int kwu_gemm_bf16_grouped_rows(const void* A, const void* B, void* C, in
                                          EpiArgs(), ga, total_rows);
   return launch_gemm<1, false, false, EPI_STORE>(bn, A, B, C, M_pad, N, K, lda, ldb, ldc, out_fp32, 0, 1.f, 0, st, status,
                                         EpiArgs(), ga, total_rows);
+}
+
+// A batch of products of one size: C[i] = alpha * A[i] op(B[i]) + diag * I, all bf16 and contiguous. A[i] (M, K) with M a
+// multiple of 128; B[i] is (N, K) with b_mn = 0 (product with its transpose) or (K, N) with b_mn = 1. Pairs of CTAs where
+// M is a multiple of 256, so that a pair's rows stay inside one matrix.
+KWU_API int kwu_gemm_bf16_batched(const void* A, const void* B, void* C, int batch, int M, int N, int K, int b_mn, float alpha,
+                                  float diag, void* stream, int* status) {
+  using namespace kwu;
+  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M % GEMM_BM) { set_last_error("gemm_bf16_batched: M must be a multiple of 128 (got %d)", M); return 7; }
+  if (static_cast<long long>(batch) * M > 0x7fffffffLL || static_cast<long long>(batch) * (b_mn ? K : N) > 0x7fffffffLL) {
+    set_last_error("gemm_bf16_batched: too many rows");
+    return 7;
+  }
+  GroupArgs ga;
+  ga.mode = 3;
+  ga.b_rows = b_mn ? K : N;
+  ga.c_rows = M;
+  ga.diag = diag;
+  const int rows = batch * M, b_rows = batch * ga.b_rows, ldb = b_mn ? N : K;
+  const TilePick pick = pick_tile(rows, N, K, b_mn != 0, false, 0, M % (2 * GEMM_BM) == 0 ? 2 : 1);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+#define KWU_BATCHED(cgv, bmn)                                                                                      \
+  if (pick.cg == cgv && (b_mn != 0) == bmn)                                                                        \
+    return launch_gemm<cgv, false, bmn, EPI_STORE>(pick.bn, A, B, C, rows, N, K, K, ldb, N, 0, 0, alpha, 0, st, status, \
+                                                   EpiArgs(), ga, b_rows)
+  KWU_BATCHED(1, false); KWU_BATCHED(1, true); KWU_BATCHED(2, false); KWU_BATCHED(2, true);
+#undef KWU_BATCHED
+  return 20;
 }
 
 // Contraction grouped by expert (weight gradients): dW[e] (N_out, K_out) (+)= dY[rows_e]^T X[rows_e].

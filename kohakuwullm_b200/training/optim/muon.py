@@ -25,12 +25,15 @@ Reference: src/kohakuwullm/training/optim/muon.py:20-107 (iterations), :178-442 
 
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
 
 from kohakuwullm_b200.ops import native
 from kohakuwullm_b200.ops.optim import adamw16_step_, sr_update_
+
+ci, cf = ctypes.c_int, ctypes.c_float
 
 NS_QUINTIC = (3.4445, -4.7750, 2.0315)
 NS_CUBIC5 = ((3.3656576, -3.3420992), (2.5744352, -1.4957376), (2.5368962, -1.4312570),
@@ -45,39 +48,49 @@ def _native_batched(a: torch.Tensor, b: torch.Tensor) -> bool:
             and a.shape[1] % 128 == 0 and a.shape[2] % 8 == 0 and b.shape[2] % 8 == 0)
 
 
-_tile_tables: dict[tuple, torch.Tensor] = {}
-
-
-def _tiles(batch: int, rows: int, device) -> torch.Tensor:
-    """Row-tile table of the grouped GEMM for ``batch`` matrices of ``rows`` rows: (first row, matrix, valid, 0)."""
-    key = (batch, rows, str(device))
-    t = _tile_tables.get(key)
-    if t is None:
-        per = rows // 128
-        m0 = torch.arange(batch * per, dtype=torch.int32) * 128
-        t = torch.stack([m0, m0 // rows, torch.ones_like(m0), torch.zeros_like(m0)], dim=1).contiguous().to(device)
-        _tile_tables[key] = t
-    return t
-
-
-def bmm_nt(a: torch.Tensor, b: torch.Tensor, b_mn: bool = False) -> torch.Tensor:
-    """Batched ``a[i] @ op(b[i])``: a (B, M, K); b (B, N, K) with ``b_mn`` false (product with b^T), or b (B, K, N)
-    with ``b_mn`` true (plain product). One grouped tcgen05 launch on a B200, ``torch.bmm`` elsewhere."""
+def bmm_nt(a: torch.Tensor, b: torch.Tensor, b_mn: bool = False, alpha: float = 1.0, diag: float = 0.0) -> torch.Tensor:
+    """Batched ``alpha * a[i] @ op(b[i]) + diag * I``: a (B, M, K); b (B, N, K) with ``b_mn`` false (product with b^T), or
+    b (B, K, N) with ``b_mn`` true (plain product). One batched tcgen05 launch on a B200, ``torch.bmm`` elsewhere."""
     B, M, K = a.shape
     N = b.shape[2] if b_mn else b.shape[1]
-    if not (_native_batched(a, b) and a.is_contiguous() and b.is_contiguous()):
-        return torch.bmm(a, b if b_mn else b.transpose(1, 2))
-    import ctypes
-
+    if not (_native_batched(a, b) and a.is_contiguous() and b.is_contiguous() and N % 8 == 0):
+        out = torch.bmm(a, b if b_mn else b.transpose(1, 2))
+        return affine(out, diag, alpha) if diag else (out if alpha == 1.0 else out * alpha)
     L = native.require()
     out = torch.empty(B, M, N, dtype=a.dtype, device=a.device)
-    tiles = _tiles(B, M, a.device)
-    ci = ctypes.c_int
-    rc = L.kwu_gemm_bf16_grouped_rows(native.ptr(a), native.ptr(b), native.ptr(out), ci(B * M), ci(N), ci(K), ci(K),
-                                      ci(b.shape[2]), ci(N), ci(int(b_mn)), ci(B), native.ptr(tiles),
-                                      ci(tiles.shape[0]), ci(0), native.ptr(None), native.stream_ptr(),
-                                      native.ptr(native.status_word()))
+    rc = L.kwu_gemm_bf16_batched(native.ptr(a), native.ptr(b), native.ptr(out), ci(B), ci(M), ci(N), ci(K), ci(int(b_mn)),
+                                 cf(alpha), cf(diag), native.stream_ptr(), native.ptr(native.status_word()))
     native.check(rc, "muon batched gemm")
+    return out
+
+
+def _native_pass(x: torch.Tensor) -> bool:
+    return x.is_cuda and x.dtype == torch.bfloat16 and native.available() and x.is_contiguous() and x.data_ptr() % 16 == 0
+
+
+def affine(gram: torch.Tensor, a: float, b: float) -> torch.Tensor:
+    """``a I + b G`` for a batch of square matrices, in one pass."""
+    n = gram.shape[-1]
+    if not (_native_pass(gram) and n % 8 == 0 and gram.numel()):
+        return torch.add(torch.eye(n, dtype=gram.dtype, device=gram.device) * a, gram, alpha=b)
+    L = native.require()
+    out = torch.empty_like(gram)
+    rc = L.kwu_diag_affine(native.ptr(gram), native.ptr(out), ci(gram.numel() // (n * n)), ci(n), cf(a), cf(b), native.stream_ptr())
+    native.check(rc, "diag_affine")
+    return out
+
+
+def scale_transpose(x: torch.Tensor, norm: torch.Tensor | None, transpose: bool) -> torch.Tensor | None:
+    """``x / norm`` (norm None: ``x``) of a bf16 (B, n, m) batch, transposed if asked, in one pass; None where the kernel
+    does not apply."""
+    B, R, C = x.shape
+    if not (_native_pass(x) and R % 2 == 0 and C % 2 == 0 and x.numel() and B <= 65535 and R <= 65535 * 64):
+        return None
+    L = native.require()
+    out = torch.empty((B, C, R) if transpose else (B, R, C), dtype=x.dtype, device=x.device)
+    rc = L.kwu_scale_transpose(native.ptr(x), native.ptr(norm), native.ptr(out), ci(B), ci(R), ci(C), ci(int(transpose)),
+                               native.stream_ptr())
+    native.check(rc, "scale_transpose")
     return out
 
 
@@ -87,8 +100,12 @@ def _prepare(grad: torch.Tensor, dtype: torch.dtype):
     says the result must be transposed back."""
     x = grad.reshape(-1, grad.shape[-2], grad.shape[-1])
     norm = torch.linalg.vector_norm(x, dim=(-2, -1), keepdim=True, dtype=torch.float32).clamp_min(1e-7) * 1.01
-    x = (x.float() / norm).to(dtype)
     transposed = x.shape[-2] > x.shape[-1]
+    if dtype == torch.bfloat16 and x.dtype == torch.bfloat16:
+        done = scale_transpose(x, norm.reshape(-1), transposed)
+        if done is not None:
+            return done, transposed
+    x = (x.float() / norm).to(dtype)
     if transposed:
         x = x.transpose(1, 2).contiguous()
     return x, transposed
@@ -96,7 +113,8 @@ def _prepare(grad: torch.Tensor, dtype: torch.dtype):
 
 def _finish(x: torch.Tensor, transposed: bool, shape) -> torch.Tensor:
     if transposed:
-        x = x.transpose(1, 2)
+        done = scale_transpose(x, None, True)     # in place of a strided view, which the write-back would walk element by element
+        x = x.transpose(1, 2) if done is None else done
     return x.reshape(shape)
 
 
@@ -119,18 +137,24 @@ def newton_schulz_cubic(grad: torch.Tensor, dtype: torch.dtype = torch.bfloat16,
     if sum(phases) != len(schedule):
         raise ValueError(f"phases {phases} sum to {sum(phases)}, the schedule has {len(schedule)} steps")
     x, transposed = _prepare(grad, dtype)
-    n = x.shape[1]
-    eye = torch.eye(n, dtype=dtype, device=x.device)
     k = 0
     for length in phases:
-        gram = bmm_nt(x, x)
-        product = None
+        product = step = gram = None
         for j in range(length):
             a, b = schedule[k + j]
-            step = torch.add(eye * a, gram, alpha=b)          # S = a I + b G (symmetric)
+            a = torch.tensor(a, dtype=x.dtype).item()         # the diagonal enters in the iteration's precision
+            # G = X X^T, then S G S; S = a I + b G (symmetric). The last S of a phase is all that its G is for, so the
+            # product that makes G writes S instead
+            if j == 0:
+                left, right, mn = x, x, False
+            else:
+                left, right, mn = bmm_nt(step, gram, b_mn=True), step, True
+            if j + 1 == length:
+                step = bmm_nt(left, right, b_mn=mn, alpha=b, diag=a)
+            else:
+                gram = bmm_nt(left, right, b_mn=mn)
+                step = affine(gram, a, b)
             product = step if product is None else bmm_nt(step, product, b_mn=True)
-            if j + 1 < length:
-                gram = bmm_nt(bmm_nt(step, gram, b_mn=True), step, b_mn=True)   # S G S
         x = bmm_nt(product, x, b_mn=True)
         k += length
     return _finish(x, transposed, grad.shape)

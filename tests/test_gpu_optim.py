@@ -137,3 +137,43 @@ def test_sumsq_flat_matches_float64_sum(n):
     assert abs(first - want) <= 2e-6 * want + 1e-12
     assert run(0) == first
     assert abs(run(1) - 2 * want) <= 4e-6 * want + 1e-12
+
+
+@pytest.mark.parametrize("batch,M,N,K", [(1, 128, 128, 64), (3, 256, 256, 72), (2, 384, 200, 136), (5, 256, 1288, 256), (2, 1280, 1280, 264)])
+def test_batched_products_with_a_diagonal(batch, M, N, K):
+    """alpha A B + d I against 64 bits: whole and cut tiles, one CTA and pairs, both storages of B. Bound: an fp32 sum of
+    K exact products is off by at most 2 K 2^-24 of the sum of magnitudes, the bf16 result by another 2^-9 of itself."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.training.optim.muon import bmm_nt
+
+    torch.manual_seed(M + N)
+    a = torch.randn(batch, M, K, device="cuda").bfloat16()
+    for mn in (False, True):
+        b = torch.randn((batch, K, N) if mn else (batch, N, K), device="cuda").bfloat16()
+        b64 = b.double() if mn else b.double().transpose(1, 2)
+        for alpha, diag in ((1.0, 0.0), (-3.25, 2.5)):
+            out = bmm_nt(a, b, b_mn=mn, alpha=alpha, diag=diag)
+            torch.cuda.synchronize()
+            native.check_status()
+            eye = torch.zeros(M, N, device="cuda", dtype=torch.float64)
+            eye.fill_diagonal_(diag)
+            want = alpha * a.double() @ b64 + eye
+            limit = 2 * K * 2.0**-24 * abs(alpha) * (a.double().abs() @ b64.abs()) + want.abs() * 2.0**-8 + 1e-6
+            assert ((out.double() - want).abs() <= limit).all()
+
+
+@pytest.mark.parametrize("batch,R,C", [(1, 2, 2), (3, 64, 66), (2, 130, 62), (2, 1792, 1280)])
+def test_scale_transpose_and_affine_equal_the_operators(batch, R, C):
+    from kohakuwullm_b200.training.optim.muon import affine, scale_transpose
+
+    torch.manual_seed(R)
+    x = torch.randn(batch, R, C, device="cuda").bfloat16()
+    norm = torch.rand(batch, device="cuda") + 0.3
+    want = (x.float() / norm[:, None, None]).bfloat16()
+    assert torch.equal(scale_transpose(x, norm, False), want)
+    assert torch.equal(scale_transpose(x, norm, True), want.transpose(1, 2))
+    assert torch.equal(scale_transpose(x, None, True), x.transpose(1, 2))
+    n = (R + 7) // 8 * 8
+    g = torch.randn(batch, n, n, device="cuda").bfloat16()
+    want = (2.5 * torch.eye(n, device="cuda", dtype=torch.float64) - 1.25 * g.double())
+    assert ((affine(g, 2.5, -1.25).double() - want).abs() <= want.abs() * 2.0**-8).all()
