@@ -84,6 +84,10 @@ struct FlashBwdParams {
 // for their tiles). K is double-buffered and loaded during the previous item, the item's first Q / dO tile is
 // loaded before its V, so the first S of an item is issued the moment the previous item's products are out,
 // and V (needed only for dP, one softmax phase later) arrives under that first phase.
+// The fp32 partials of a key tile leave through shared memory and TMA, 128-byte row segments at a time: as one 16-byte
+// store per lane and row they were a quarter of the kernel on short documents and windows (4096-token packs 78 us of
+// which 17, 66 with TMA; 16384 tokens with a window of 1024 317 us of which 77, 253 with TMA). The buffers that hold the
+// item's V and K are free for that once its products are done; a warp whose rows reach past the document stores directly.
 constexpr int FBK_STAGES = 3;
 constexpr int FBK_SMEM = 3 * 16384 + FBK_STAGES * 16384 + 2048 + 1024 + 1024;
 
@@ -107,6 +111,7 @@ __device__ __forceinline__ bool dkdv_decode(const FlashBwdParams& p, int item, D
 __global__ void __launch_bounds__(FB_THREADS, 2)
 flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmDO64,
                       const __grid_constant__ CUtensorMap tmK128, const __grid_constant__ CUtensorMap tmV128,
+                      const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
                       const FlashBwdParams p) {
   pdl_sync();   // nothing of the previous kernel is read above this line
   extern __shared__ uint8_t smem_raw[];
@@ -120,14 +125,14 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
   float* sDelta = sLse + FBK_STAGES * 64;                                      // per stage 64: -delta * scale
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 49152 + FBK_STAGES * 16384 + 2048);
   uint64_t* k_full = bars + 0;    // [2]
-  uint64_t* k_empty = bars + 2;   // [2] the item's last products have read this K buffer
+  uint64_t* k_empty = bars + 2;   // [2] the item's last products, and the output staged there, have left this K buffer
   uint64_t* qd_full = bars + 4;   // [3]
   uint64_t* qd_empty = bars + 7;  // [3]
   uint64_t* sdp_full = bars + 10;
   uint64_t* p_ready = bars + 11;
   uint64_t* acc_done = bars + 12;
   uint64_t* v_full = bars + 13;
-  uint64_t* v_empty = bars + 14;   // the item's last products have read V
+  uint64_t* v_empty = bars + 14;   // the same of V
   uint64_t* acc_free = bars + 15;  // the item's dK / dV accumulators have been read out
   uint64_t* dp_full = bars + 16;   // dP^T is in TMEM (S^T has its own barrier, so the exponentials start earlier)
   uint64_t* ds_ready = bars + 17;  // dS^T has been written (P^T has its own barrier, so dV starts earlier)
@@ -141,10 +146,10 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
+      mbar_init(&k_empty[s], 1 + 4);   // the products' commit and the four warps that stage their output there
     }
     mbar_init(v_full, 1);
-    mbar_init(v_empty, 1);
+    mbar_init(v_empty, 1 + 4);
     for (int s = 0; s < FBK_STAGES; ++s) {
       mbar_init(&qd_full[s], 1);
       mbar_init(&qd_empty[s], 1);
@@ -464,7 +469,30 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
         tmem_ld_wait();
         tc_fence_before();
         mbar_arrive_warp(acc_free);   // the next item's first products may overwrite the accumulators now
-        if (kj < de) {
+        const int row0 = it.kv0 + quarter * 32;      // first key of this warp
+        if (p.dk_part && row0 + 32 <= de) {
+          uint8_t* patch = (which == 0 ? sV : sK + (ic & 1) * 16384) + quarter * 4096;
+          const CUtensorMap* tm = which == 0 ? &tmDV : &tmDK;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            if (c == 1) {
+              if (lane == 0) tma_store_wait_read<0>();
+              __syncwarp();
+            }
+            // 128-byte rows, 16-byte units XORed with the row (the TMA's 128-byte swizzle)
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+              *reinterpret_cast<uint4*>(patch + lane * 128 + ((v ^ (lane & 7)) << 4)) =
+                  make_uint4(o[c * 32 + 4 * v], o[c * 32 + 4 * v + 1], o[c * 32 + 4 * v + 2], o[c * 32 + 4 * v + 3]);
+            fence_async_proxy();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(tm, patch, h * FB_D + c * 32, row0);
+              tma_store_commit();
+            }
+          }
+          if (lane == 0) tma_store_wait_read<0>();
+        } else if (kj < de) {
           if (p.dk_part) {
             float4* dst = reinterpret_cast<float4*>((which == 0 ? p.dv_part : p.dk_part) +
                                                     (static_cast<size_t>(kj) * p.Hq + h) * FB_D);
@@ -488,6 +516,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
           }
         }
       }
+      mbar_arrive_warp(half == 0 ? v_empty : &k_empty[ic & 1]);   // staged output (if any) has been read
       g += it.n_it;
       ++ic;
     }
@@ -888,7 +917,12 @@ KWU_API int kwu_flash_bwd(const void* q, int q_ld, const void* k, int k_ld, cons
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long items = static_cast<long long>(n_tiles) * Hq;
   const int pgrid = static_cast<int>(items < 2LL * sms ? items : 2LL * sms);   // two resident CTAs per SM walk the items
-  launch_k(flash_bwd_dkdv_kernel, dim3(pgrid), dim3(FB_THREADS), FBK_SMEM, st, tmQ64, tmDO64, tmK128, tmV128, p); kwu::count_launch();
+  CUtensorMap tmDK = tmK128, tmDV = tmV128;   // not read without partials
+  if (p.dk_part) {
+    if ((rc = encode_tmap_2d(&tmDK, p.dk_part, ELEM_F32, T, wq, wq, 32, 32, SW))) return rc;
+    if ((rc = encode_tmap_2d(&tmDV, p.dv_part, ELEM_F32, T, wq, wq, 32, 32, SW))) return rc;
+  }
+  launch_k(flash_bwd_dkdv_kernel, dim3(pgrid), dim3(FB_THREADS), FBK_SMEM, st, tmQ64, tmDO64, tmK128, tmV128, tmDK, tmDV, p); kwu::count_launch();
   if (Hq > Hkv) {
     long g = (static_cast<long>(T) * Hkv * 16 + 255) / 256;
     if (g > 148 * 16) g = 148 * 16;
