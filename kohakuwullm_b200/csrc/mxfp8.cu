@@ -74,7 +74,10 @@ mxfp8_quantize_kernel(const __nv_bfloat16* __restrict__ x, int ldx, uint8_t* __r
 }
 
 // Transposed quantise: input (R, C) row-major, output qT (C, R) with blocks of 32 along R.
-// A block handles a 32 (rows) x 64 (cols) input tile: thread t < 64 owns column c0 + t.
+// A block handles a 32 (rows) x 64 COLS (columns) input tile; thread t owns the COLS columns from COLS t. With two, a warp
+// reads whole 128-byte lines in half as many loads; rows that are not 4-byte aligned pairs take one. us, one / two columns:
+// 1280 x 3584 (mean of a layer's matrices) 9.0 / 6.2, 64 experts of 768 x 1024 20.4 / 12.2.
+template <int COLS>
 __global__ void __launch_bounds__(64)
 mxfp8_quantize_t_kernel(const __nv_bfloat16* __restrict__ x, int ldx, uint8_t* __restrict__ qT, int ldq,
                         uint8_t* __restrict__ sf, int R, int C, int C_pad, long long x_batch, long long q_batch,
@@ -85,37 +88,56 @@ mxfp8_quantize_t_kernel(const __nv_bfloat16* __restrict__ x, int ldx, uint8_t* _
   qT += static_cast<size_t>(blockIdx.z) * q_batch;
   sf += static_cast<size_t>(blockIdx.z) * sf_batch;
   const int r0 = blockIdx.y * 32;
-  const int c = blockIdx.x * 64 + threadIdx.x;
-  if (c >= C_pad) return;
+  const int c0 = (blockIdx.x * 64 + threadIdx.x) * COLS;
+  if (c0 >= C_pad) return;
   const int n_kchunks = (R + 127) >> 7;  // contraction axis of the output is R
-  float v[32];
-  float amax = 0.f;
+  uint32_t raw[32];                      // one bf16 in the low half, or the pair of two columns
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     const int r = r0 + i;
-    v[i] = (r < R && c < C) ? __bfloat162float(x[static_cast<size_t>(r) * ldx + c]) : 0.f;
-    amax = fmaxf(amax, fabsf(v[i]));
+    raw[i] = 0u;
+    if (r < R && c0 < C) {               // with two columns C is even: a pair is inside or outside
+      const __nv_bfloat16* at = x + static_cast<size_t>(r) * ldx + c0;
+      raw[i] = COLS == 2 ? *reinterpret_cast<const uint32_t*>(at) : *reinterpret_cast<const uint16_t*>(at);
+    }
   }
-  const uint32_t e8 = (c < C) ? ue8m0_from_amax(amax) : 127u;
-  if (r0 < R && (sf_bn <= 128 || c < C)) sf[sf_offset_any(c, r0 >> 5, n_kchunks, sf_bn)] = static_cast<uint8_t>(e8);
-  if (c < C) {
-    const float inv = inv_scale_from_ue8m0(e8);
-    uint32_t w[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const __nv_fp8x2_storage_t a2 = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] * inv, v[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-      const __nv_fp8x2_storage_t b2 = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j + 2] * inv, v[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-      w[j] = static_cast<uint32_t>(a2) | (static_cast<uint32_t>(b2) << 16);
-    }
-    uint4* dst = reinterpret_cast<uint4*>(qT + static_cast<size_t>(c) * ldq + r0);
-    if (r0 + 32 <= R) {
-      dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-      dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    } else {
-      uint8_t* d8 = qT + static_cast<size_t>(c) * ldq + r0;
-      for (int i = 0; i < 32 && r0 + i < R; ++i) d8[i] = static_cast<uint8_t>(w[i >> 2] >> (8 * (i & 3)));
+  for (int k = 0; k < COLS; ++k) {
+    const int c = c0 + k;
+    auto value = [&](int i) { return __uint_as_float(k == 0 ? raw[i] << 16 : raw[i] & 0xffff0000u); };
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(value(i)));
+    const uint32_t e8 = (c < C) ? ue8m0_from_amax(amax) : 127u;
+    if (r0 < R && (sf_bn <= 128 || c < C)) sf[sf_offset_any(c, r0 >> 5, n_kchunks, sf_bn)] = static_cast<uint8_t>(e8);
+    if (c < C) {
+      const float inv = inv_scale_from_ue8m0(e8);
+      uint32_t w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const __nv_fp8x2_storage_t a2 = __nv_cvt_float2_to_fp8x2(make_float2(value(4 * j) * inv, value(4 * j + 1) * inv), __NV_SATFINITE, __NV_E4M3);
+        const __nv_fp8x2_storage_t b2 = __nv_cvt_float2_to_fp8x2(make_float2(value(4 * j + 2) * inv, value(4 * j + 3) * inv), __NV_SATFINITE, __NV_E4M3);
+        w[j] = static_cast<uint32_t>(a2) | (static_cast<uint32_t>(b2) << 16);
+      }
+      uint4* dst = reinterpret_cast<uint4*>(qT + static_cast<size_t>(c) * ldq + r0);
+      if (r0 + 32 <= R) {
+        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      } else {
+        uint8_t* d8 = qT + static_cast<size_t>(c) * ldq + r0;
+        for (int i = 0; i < 32 && r0 + i < R; ++i) d8[i] = static_cast<uint8_t>(w[i >> 2] >> (8 * (i & 3)));
+      }
     }
   }
+}
+
+static void launch_quantize_t(const void* x, int ldx, void* qT, int ldq, void* sf, int R, int C, int C_pad, int batch,
+                              long long x_batch, long long q_batch, long long sf_batch, int sf_bn, cudaStream_t st) {
+  const bool pairs = C % 2 == 0 && ldx % 2 == 0 && x_batch % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+  const int cols = pairs ? 128 : 64;
+  launch_k(pairs ? mxfp8_quantize_t_kernel<2> : mxfp8_quantize_t_kernel<1>, dim3((C_pad + cols - 1) / cols, R / 32, batch), dim3(64), 0, st,
+           (const __nv_bfloat16*)x, ldx, (uint8_t*)qT, ldq, (uint8_t*)sf, R, C, C_pad, x_batch, q_batch, sf_batch, sf_bn);
+  kwu::count_launch();
 }
 
 // ------------------------------------------------------------------------------------ GEMM
@@ -592,9 +614,7 @@ KWU_API int kwu_mxfp8_quantize_t(const void* x, int ldx, void* qT, int ldq, void
   if (R % 128) { set_last_error("mxfp8_quantize_t: R must be a multiple of 128 (got %d)", R); return 7; }
   if (C <= 0) return 0;
   const int C_pad = (C + 127) / 128 * 128;
-  dim3 grid((C_pad + 63) / 64, R / 32);
-  launch_k(mxfp8_quantize_t_kernel, dim3(grid), dim3(64), 0, reinterpret_cast<cudaStream_t>(stream), 
-      (const __nv_bfloat16*)x, ldx, (uint8_t*)qT, ldq, (uint8_t*)sf, R, C, C_pad, 0, 0, 0, 0); kwu::count_launch();
+  launch_quantize_t(x, ldx, qT, ldq, sf, R, C, C_pad, 1, 0, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error("mxfp8_quantize_t launch: %s", cudaGetErrorString(e)); return 11; }
   return 0;
@@ -630,9 +650,7 @@ KWU_API int kwu_mxfp8_quantize_t_w(const void* x, int ldx, void* qT, int ldq, vo
   if (!bn_supported(sf_bn)) { set_last_error("mxfp8_quantize_t_w: unsupported tile width %d", sf_bn); return 7; }
   if (C <= 0) return 0;
   const int C_pad = (C + 127) / 128 * 128;
-  dim3 grid((C_pad + 63) / 64, R / 32);
-  launch_k(mxfp8_quantize_t_kernel, dim3(grid), dim3(64), 0, reinterpret_cast<cudaStream_t>(stream), 
-      (const __nv_bfloat16*)x, ldx, (uint8_t*)qT, ldq, (uint8_t*)sf, R, C, C_pad, 0, 0, 0, sf_bn); kwu::count_launch();
+  launch_quantize_t(x, ldx, qT, ldq, sf, R, C, C_pad, 1, 0, 0, 0, sf_bn, reinterpret_cast<cudaStream_t>(stream));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error("mxfp8_quantize_t_w launch: %s", cudaGetErrorString(e)); return 11; }
   return 0;
@@ -644,10 +662,8 @@ KWU_API int kwu_mxfp8_quantize_t_batched(const void* x, int ldx, void* qT, int l
                                          void* stream) {
   if (R % 128 || C % 128) { set_last_error("mxfp8_quantize_t_batched: R and C must be multiples of 128"); return 7; }
   if (batch <= 0) return 0;
-  dim3 grid(C / 64, R / 32, batch);
-  launch_k(mxfp8_quantize_t_kernel, dim3(grid), dim3(64), 0, reinterpret_cast<cudaStream_t>(stream), 
-      (const __nv_bfloat16*)x, ldx, (uint8_t*)qT, ldq, (uint8_t*)sf, R, C, C, static_cast<long long>(R) * ldx,
-      static_cast<long long>(C) * ldq, kwu_mxfp8_sf_bytes(C, R), 0); kwu::count_launch();
+  launch_quantize_t(x, ldx, qT, ldq, sf, R, C, C, batch, static_cast<long long>(R) * ldx, static_cast<long long>(C) * ldq,
+                    kwu_mxfp8_sf_bytes(C, R), 0, reinterpret_cast<cudaStream_t>(stream));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error("mxfp8_quantize_t_batched launch: %s", cudaGetErrorString(e)); return 11; }
   return 0;

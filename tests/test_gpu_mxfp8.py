@@ -257,3 +257,17 @@ def test_gemm_tile_widths_and_outputs(M, N, K, bn):
             native.check_status()
             limit = bound + want.abs() * (2.0**-23 if dtype == torch.float32 else 2.0**-8)
             assert ((out.double() - want).abs() <= limit).all(), f"{dtype} accumulate {accumulate}"
+
+
+@pytest.mark.parametrize("R,C,offset", [(128, 1, 0), (128, 62, 1), (256, 63, 0), (384, 130, 0), (128, 257, 3), (256, 1280, 2)])
+def test_transposed_quantise_of_odd_and_unaligned_matrices(R, C, offset):
+    """Pairs of columns per thread or one, by alignment: the same bytes as quantising the transposed copy."""
+    from kohakuwullm_b200.ops import mxfp8 as mx
+
+    torch.manual_seed(C)
+    store = (torch.randn(R, C + 8, device="cuda") * torch.logspace(-4, 3, R, device="cuda")[:, None]).to(torch.bfloat16)
+    w = store[:, offset:offset + C]
+    qt, sft = mx.quantize_transposed(w)
+    q_ref, e_ref = mx.quantize_reference(w.t().contiguous())
+    assert torch.equal(qt.view(torch.float8_e4m3fn).float(), q_ref.float())
+    assert torch.equal(mx.sf_to_natural(sft, C, R), e_ref)
