@@ -69,6 +69,9 @@ struct GemmParams {
   // would leave the last round of the persistent grid partly empty, is cut into `splits` ranges of the contraction for
   // CTAs (pairs) that would idle, all adding into C. 0 tail tiles: every tile is a whole item.
   int full_tiles, tail_tiles, splits;
+  // even ranges (single CTAs, fp32 C += only): the (tile, k-block) units, tiles row by row, are cut into this many equal
+  // contiguous ranges, one per CTA; every tile is the sum of the pieces of the ranges that meet in it. 0: off.
+  int ranges;
   // grouped (mixture-of-experts) modes
   //   1: rows grouped by expert: row tile t reads group_tiles[t] = (m0, expert, valid); the expert picks
   //      a block of `group_b_rows` rows of B (K-major: output rows; MN-major: contraction rows)
@@ -163,6 +166,23 @@ __device__ __forceinline__ bool decode_tile(const GemmParams& p, int tile, int n
 // Work item number `i` of this CTA (pair). 0: none left; 1: `t` holds work; 2: nothing to do for this index, go on.
 template <int CG>
 __device__ __forceinline__ int next_work(const GemmParams& p, int i, int num_tiles, int num_kb, TileInfo& t) {
+  if (CG == 1 && p.ranges > 0) {
+    const long long units = static_cast<long long>(num_tiles) * num_kb;
+    const long long u0 = units * blockIdx.x / p.ranges, u1 = units * (blockIdx.x + 1) / p.ranges;
+    // the piece that begins its tile first, then the one that ends its tile: with about one tile per range every CTA then
+    // walks the contraction from 0 to K at the same time as the others, and the slabs of A and B that they share stay in
+    // the L2 (tile by tile the ranges are spread over the whole contraction)
+    const long long first = u0 / num_kb, pieces = u1 > u0 ? (u1 - 1) / num_kb - first + 1 : 0;
+    if (i >= pieces) return 0;
+    const long long tile = i == 0 ? first + pieces - 1 : first + i - 1;
+    const long long start = max(u0, tile * num_kb), end = min(u1, (tile + 1) * num_kb);
+    t.b_row_off = 0; t.c_row_off = 0;
+    t.m0 = static_cast<int>(tile / p.tiles_n) * GEMM_BM;
+    t.n0 = static_cast<int>(tile % p.tiles_n) * p.bn;
+    t.k_begin = static_cast<int>(start - tile * num_kb) * GEMM_BK;
+    t.nkb = static_cast<int>(end - start);
+    return 1;
+  }
   const int item = static_cast<int>(blockIdx.x) / CG + i * (static_cast<int>(gridDim.x) / CG);
   if (p.tail_tiles > 0 && item >= p.full_tiles) {
     const int piece = item - p.full_tiles;
@@ -676,7 +696,7 @@ template <int CG, bool A_MN, bool B_MN, int EPI>
 static int launch_gemm(int BN, const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                        int ldc, int out_fp32, int accumulate, float alpha, int max_ctas,
                        cudaStream_t stream, int* status, const EpiArgs& ea = EpiArgs(),
-                       const GroupArgs& ga = GroupArgs(), int b_total_rows = 0, int splits = 1) {
+                       const GroupArgs& ga = GroupArgs(), int b_total_rows = 0, int splits = 1, bool even_ranges = false) {
   CUtensorMap tmA, tmB, tmC;
   int rc;
   if (!A_MN)
@@ -756,7 +776,13 @@ static int launch_gemm(int BN, const void* A, const void* B, void* C, int M, int
     p.splits = splits;
   }
   const long items = p.full_tiles + static_cast<long>(p.tail_tiles) * p.splits;
-  if (items < units) units = static_cast<int>(items);
+  p.ranges = 0;
+  if (CG == 1 && even_ranges && ga.mode == 0 && out_fp32 && accumulate && EPI == EPI_STORE) {
+    const long long all = tiles * static_cast<long long>((K + GEMM_BK - 1) / GEMM_BK);
+    p.ranges = units = static_cast<int>(all < units ? all : units);
+  } else if (items < units) {
+    units = static_cast<int>(items);
+  }
   const size_t smem = 1024 + GEMM_BAR_BYTES + GEMM_OUT_BYTES + static_cast<size_t>(p.stages) * p.stage_bytes;
   launch_cluster(kern, dim3(units * CG), dim3(GEMM_THREADS), CG, smem, stream, tmA, tmB, tmC, C, p); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
@@ -831,6 +857,14 @@ KWU_API int kwu_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   }
   TilePick pick{bn > 1000 ? 2 : 1, bn > 1000 ? bn - 1000 : bn, 1};
   if (bn == 0) pick = pick_tile(M, N, K, b_mn != 0, out_fp32 && accumulate, 0, 2, max_ctas);
+  // dx += dy W with a long contraction is the loss head's input gradient, 65536 deep, on which every layer's gradient
+  // rests: rounded to bf16 and re-quantised to e4m3 below, one bit of its sums becomes several percent of noise in the
+  // gradients of the first layers. So its sums stay cut the way they always were, into one even range of 128 x 256 tiles'
+  // k-blocks per SM: 4096 x 1280 x 65536 in 489 us (683 with the ranges walked tile by
+  // tile and per-lane additions, 437 on pairs).
+  const bool even = bn == 0 && out_fp32 && accumulate && !a_mn && b_mn && K >= 1024 &&
+                    (static_cast<long>((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256)) % num_sms() != 0;
+  if (even) pick = {1, 256, 1};
   if (pick.bn < 64 || pick.bn > 256 || pick.bn % 32) {
     set_last_error("kwu_gemm_bf16: tile width %d", pick.bn);
     return 20;
@@ -839,7 +873,7 @@ KWU_API int kwu_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   if (pick.cg == cgv && a_mn == amn && b_mn == bmn)                                               \
     return launch_gemm<cgv, amn != 0, bmn != 0, EPI_STORE>(pick.bn, A, B, C, M, N, K, lda, ldb, ldc, out_fp32,        \
                                                 accumulate, alpha, max_ctas, st, status, EpiArgs(), \
-                                                GroupArgs(), 0, pick.splits);
+                                                GroupArgs(), 0, pick.splits, even);
   KWU_GEMM_CASE(1, 0, 0) KWU_GEMM_CASE(1, 0, 1) KWU_GEMM_CASE(1, 1, 0) KWU_GEMM_CASE(1, 1, 1)
   KWU_GEMM_CASE(2, 0, 0) KWU_GEMM_CASE(2, 0, 1) KWU_GEMM_CASE(2, 1, 0) KWU_GEMM_CASE(2, 1, 1)
 #undef KWU_GEMM_CASE
@@ -891,43 +925,47 @@ KWU_API int kwu_gemm_dlogits(const void* H, const void* W, void* dlogits, int T,
 }
 
 namespace kwu {
-// 32 rows by 8 slices of the column tiles per block: a thread folds every eighth partial of its row (a warp reads 256
-// contiguous bytes), then the slices are folded in shared memory. One thread per row alone left 64 of 148 SMs with
-// one chain of 256 dependent loads each (40 us at 8190 rows and 256 tiles; 6 us like this).
-constexpr int CE_ROWS = 32, CE_SLICES = 8;
-__global__ void __launch_bounds__(CE_ROWS * CE_SLICES) ce_combine_kernel(const float2* __restrict__ partial, int tiles_n, int M,
-                                                                         float* __restrict__ lse) {
-  __shared__ float2 part[CE_SLICES][CE_ROWS];
-  const int r = threadIdx.x % CE_ROWS, sl = threadIdx.x / CE_ROWS;
-  const int row = blockIdx.x * CE_ROWS + r;
+// One thread folds a row's partials in order of the tiles (every gradient of the step rests on the last bit of this sum
+// through bf16 and e4m3 roundings, so its order stays). A block is one warp, so that 4096 rows reach 128 SMs, and a batch
+// of partials is fetched ahead of its use: 128 rows a block and one load behind the other took 40 us at 8190 rows and 256
+// tiles, 13 like this (6 with the tiles folded in slices).
+constexpr int CE_ROWS = 32, CE_AHEAD = 32;
+__global__ void __launch_bounds__(CE_ROWS) ce_combine_kernel(const float2* __restrict__ partial, int tiles_n, int M,
+                                                             float* __restrict__ lse) {
+  const int row = blockIdx.x * CE_ROWS + threadIdx.x;
+  if (row >= M) return;
   float m = -INFINITY, s = 0.f;
-  if (row < M) {
-    for (int t = sl; t < tiles_n; t += CE_SLICES) {
-      const float2 v = partial[static_cast<size_t>(t) * M + row];
-      const float nm = fmaxf(m, v.x);
-      s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
-      m = nm;
-    }
-  }
-  part[sl][r] = make_float2(m, s);
-  __syncthreads();
-  if (sl == 0 && row < M) {
+  auto fold = [&](const float2& v) {
+    const float nm = fmaxf(m, v.x);
+    s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
+    m = nm;
+  };
+  const float2* at = partial + row;
+  const int whole = tiles_n / CE_AHEAD * CE_AHEAD;
+  float2 next[CE_AHEAD];
+  if (whole) {
 #pragma unroll
-    for (int i = 1; i < CE_SLICES; ++i) {
-      const float2 v = part[i][r];
-      if (v.x == -INFINITY) continue;      // a slice without a tile
-      const float nm = fmaxf(m, v.x);
-      s = s * __expf(m - nm) + v.y * __expf(v.x - nm);
-      m = nm;
-    }
-    lse[row] = m + __logf(s);
+    for (int i = 0; i < CE_AHEAD; ++i) next[i] = at[static_cast<size_t>(i) * M];
   }
+  for (int t0 = 0; t0 < whole; t0 += CE_AHEAD) {
+    float2 now[CE_AHEAD];
+#pragma unroll
+    for (int i = 0; i < CE_AHEAD; ++i) now[i] = next[i];
+    if (t0 + CE_AHEAD < whole) {
+#pragma unroll
+      for (int i = 0; i < CE_AHEAD; ++i) next[i] = at[static_cast<size_t>(t0 + CE_AHEAD + i) * M];
+    }
+#pragma unroll
+    for (int i = 0; i < CE_AHEAD; ++i) fold(now[i]);
+  }
+  for (int t = whole; t < tiles_n; ++t) fold(at[static_cast<size_t>(t) * M]);
+  lse[row] = m + __logf(s);
 }
 }  // namespace kwu
 
 KWU_API int kwu_ce_combine(const void* partial, int tiles_n, int M, float* lse, void* stream) {
   if (M <= 0) return 0;
-  kwu::ce_combine_kernel<<<(M + kwu::CE_ROWS - 1) / kwu::CE_ROWS, kwu::CE_ROWS * kwu::CE_SLICES, 0,
+  kwu::ce_combine_kernel<<<(M + kwu::CE_ROWS - 1) / kwu::CE_ROWS, kwu::CE_ROWS, 0,
                            reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const float2*>(partial), tiles_n, M, lse); kwu::count_launch();
   cudaError_t e = cudaGetLastError();
