@@ -104,7 +104,7 @@ def test_gemm_tile_widths_and_cta_pairs(shape, a_mn, b_mn, bn):
 
 @pytest.mark.parametrize("vocab", [1000, 256 * 9])
 def test_cross_entropy_partials_fold(vocab):
-    """Column tiles that do not fill the eight slices of the folding kernel, and rows that end inside its block."""
+    """Column tiles that are no whole batch of the folding kernel, and rows that end inside its block."""
     from kohakuwullm_b200.ops.loss import linear_cross_entropy, linear_cross_entropy_reference
 
     g = torch.Generator(device="cuda").manual_seed(vocab)
@@ -138,3 +138,40 @@ def test_few_rows_against_64_bits(M, N, K, out_dtype):
     limit = K * 2.0**-24 * (a.double().abs() @ b.double().abs().t()) + want.abs() * (2.0**-8 if out_dtype == torch.bfloat16 else 2.0**-23) + 1e-7
     assert ((out.double() - want).abs() <= limit).all()
     assert (store[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 64, 1024), (130, 264, 1096), (300, 520, 4104), (640, 1280, 8192), (4096, 1280, 2056), (2500, 2600, 1024)])
+def test_input_gradient_sums_in_even_ranges(M, N, K):
+    """fp32 C += A B with B contraction-major and a long contraction: fewer tiles than SMs (several ranges meet in a tile),
+    about one each, and more; cut tiles and contractions. Bound: fp32 sums of K exact products, at most 2 K 2^-24 of the sum
+    of magnitudes, plus the rounding of a few pieces."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.gemm import matmul
+
+    torch.manual_seed(K)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = torch.randn(K, N, device="cuda").bfloat16()
+    out = torch.randn(M, N, device="cuda")
+    want = out.double() + a.double() @ b.double()
+    limit = 2 * K * 2.0**-24 * (a.double().abs() @ b.double().abs()) + want.abs() * 2.0**-20 + 1e-5
+    matmul(a, b, b_mn=True, out=out, accumulate=True)
+    torch.cuda.synchronize()
+    native.check_status()
+    assert ((out.double() - want).abs() <= limit).all()
+
+
+@pytest.mark.parametrize("tiles", [1, 31, 32, 33, 64, 65, 256])
+def test_fold_of_cross_entropy_partials_around_a_batch(tiles):
+    """Whole batches of partials, none and a remainder; the fold's error is a few fp32 roundings."""
+    import ctypes
+
+    from kohakuwullm_b200.ops import native
+
+    torch.manual_seed(tiles)
+    rows = 77
+    part = torch.stack([torch.randn(tiles, rows, device="cuda") * 8, torch.rand(tiles, rows, device="cuda") * 50 + 1], -1).contiguous()
+    lse = torch.empty(rows, device="cuda")
+    rc = native.require().kwu_ce_combine(native.ptr(part), ctypes.c_int(tiles), ctypes.c_int(rows), native.ptr(lse), native.stream_ptr())
+    native.check(rc, "ce_combine")
+    want = torch.logsumexp(part[..., 0].double() + part[..., 1].double().log(), 0)
+    assert ((lse.double() - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
