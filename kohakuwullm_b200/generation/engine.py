@@ -99,7 +99,8 @@ class StepGraph:
         self.graph = torch.cuda.CUDAGraph()
         length = cache.length
         cache.hold_position(token.device)
-        stream = torch.cuda.Stream(device=token.device)
+        # the memory of a capture belongs to its stream: the next capture can take it over only there
+        self.stream = stream = torch.cuda.Stream(device=token.device) if earlier is None else earlier.stream
         stream.wait_stream(torch.cuda.current_stream(token.device))
         try:
             with torch.cuda.stream(stream):
