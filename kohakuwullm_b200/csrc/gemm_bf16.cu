@@ -856,7 +856,11 @@ KWU_API int kwu_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
     return 0;
   }
   TilePick pick{bn > 1000 ? 2 : 1, bn > 1000 ? bn - 1000 : bn, 1};
-  if (bn == 0) pick = pick_tile(M, N, K, b_mn != 0, out_fp32 && accumulate, 0, 2, max_ctas);
+  // The pieces of a cut tile meet in C in the order in which they finish, so a cut costs the fixed order of the sum. Below
+  // K = 1024 no tile is cut: it would save at most a few microseconds, and callers rest on the order there (the gate logits
+  // of routed layers up to 1023 wide, head plus remainder of the gate matrix: near ties between experts would fall
+  // differently from run to run).
+  if (bn == 0) pick = pick_tile(M, N, K, b_mn != 0, out_fp32 && accumulate && K >= 1024, 0, 2, max_ctas);
   // dx += dy W with a long contraction is the loss head's input gradient, 65536 deep, on which every layer's gradient
   // rests: rounded to bf16 and re-quantised to e4m3 below, one bit of its sums becomes several percent of noise in the
   // gradients of the first layers. So its sums stay cut the way they always were, into one even range of 128 x 256 tiles'

@@ -175,3 +175,25 @@ def test_fold_of_cross_entropy_partials_around_a_batch(tiles):
     native.check(rc, "ce_combine")
     want = torch.logsumexp(part[..., 0].double() + part[..., 1].double().log(), 0)
     assert ((lse.double() - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 768), (17, 64, 768), (3001, 64, 768), (8190, 64, 768), (640, 1280, 1016), (300, 64, 1000)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+def test_short_contractions_add_into_fp32_in_one_piece(M, N, K, a_mn, b_mn):
+    """fp32 C += A B below K = 1024 has one order of summation: it is C plus the product that the same tile writes without
+    accumulation, to the bit, however often it runs (gate logits of routed layers are formed like this)."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.gemm import matmul
+
+    if a_mn and M % 8:
+        M = (M + 7) // 8 * 8           # pitches of TMA operands
+    a, b, _ = _operands(M, N, K, a_mn, b_mn, seed=K)
+    start = torch.randn(M, N, device="cuda")
+    # bn = 128: the plain tile kernel for every M
+    product = matmul(a, b, a_mn=a_mn, b_mn=b_mn, bn=128, out_dtype=torch.float32)
+    for _ in range(4):
+        out = start.clone()
+        matmul(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=True)
+        assert torch.equal(out, start + product)
+    torch.cuda.synchronize()
+    native.check_status()
