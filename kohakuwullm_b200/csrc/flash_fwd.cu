@@ -13,10 +13,14 @@
 // 53.3 -> 50.5 us, 16384 tokens with a window of 1024 227 -> 218; one long document is bound by the exponentials either
 // way (1316 us, 735 of them at the special-function rate, 1068 without them).
 //
-// SPLIT (cached prefill and other padded batches, which keep 32-bit probabilities): P leaves the softmax as two bf16
-// numbers, its rounding and what the rounding left out (together 16 bits of mantissa and more), and O += P V runs once
-// for each. The low parts overwrite score columns that the same thread has read, so the low product is issued before
-// the next tile's scores and the high one after them: the tensor pipe stays ahead of the softmax, which is the bound.
+// SPLIT (cached prefill and other padded batches, which keep 32-bit probabilities): P leaves the softmax as three bf16
+// numbers, its rounding, the rounding of what that left out, and the rest: 8 + 8 + 8 bits hold an fp32 number exactly, and
+// O += P V runs once for each. The two lower parts overwrite score columns that the same thread has read, so their
+// products are issued before the next tile's scores and the high one after them: the tensor pipe stays ahead of the
+// softmax, which is the bound. On sums that cancel, two parts (16 bits) were 10 to 20 times as far from 64 bits as the
+// explicit fp32 form; three are nearer than it inside one key tile, and 2e-7 of the sum of magnitudes off over 3001 keys
+// (2e-8 the explicit form), where the tensor pipe's own fp32 sums are what is left. On ordinary values both forms' errors
+// are the output's bf16 rounding and agree to 1e-6. The third part costs two prompts of 3001 tokens 0.55 of 10.0 ms.
 //
 // Documents never attend across their boundary: a tile's key range is clipped to its own document
 // and (with a window) to the last `window` positions. Sinks enter as sink_lse[h] = logsumexp of the
@@ -139,7 +143,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* o_done = bars + 11;
   uint64_t* q_empty = bars + 12;  // the item's last S product has read Q
   uint64_t* o_free = bars + 13;   // the softmax warps have read the item's O accumulator
-  uint64_t* s_free = bars + 14;   // the scores of a tile are in registers (not SPLIT, which keeps P's low parts there)
+  uint64_t* s_free = bars + 14;   // the scores of a tile are in registers (not SPLIT, which keeps P's lower parts there)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_rowmax = reinterpret_cast<float*>(smem + 5 * FA_TILE_BYTES + 1024);  // 2 x 256 max + 256 sums
@@ -274,11 +278,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         tc_fence_after();
         if (SPLIT) {
-          // low parts: the first 32 of each thread's 64 score columns (keys 64 h .. 64 h + 63 at columns 64 h .. 64 h + 31)
+          // keys 32 i .. 32 i + 31: middle parts at score columns 32 i .. 32 i + 15, low parts at the 16 after them
           if (leader) {
 #pragma unroll
-            for (int k = 0; k < FA_BN / 16; ++k)
-              mma_f16_ts(tO, tS + (k >> 2) * 64 + (k & 3) * 8, dV + 128 * k, idesc_o, k > 0 ? 1u : acc);
+            for (int part = 1; part >= 0; --part)
+#pragma unroll
+              for (int k = 0; k < FA_BN / 16; ++k)
+                mma_f16_ts(tO, tS + (k >> 1) * 32 + part * 16 + (k & 1) * 8, dV + 128 * k, idesc_o, k > 0 || part == 0 ? 1u : acc);
           }
           __syncwarp();
           acc = 1u;
@@ -365,9 +371,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         pair_sync();
         mx = fmaxf(fmaxf(mx, xbuf[(half ^ 1) * 128 + row]), m);
         if (!ok) continue;
-        const float alpha = fast_exp2((m - mx) * p.scale_log2);
+        const float neg_ms = __fmul_rn(-mx, p.scale_log2);
+        // SPLIT: from the rounded products that the exponents are taken against, so that keys of different tiles keep their
+        // ratio to the last bits
+        const float alpha = fast_exp2(SPLIT ? neg_ms + __fmul_rn(m, p.scale_log2) : (m - mx) * p.scale_log2);
         m = mx;
-        const float neg_ms = -mx * p.scale_log2;
         // the previous P V product must be complete before P is overwritten and O is touched; for the
         // first tile of an item that product belongs to the previous item and was waited for in its epilogue
         if (j > 0) {
@@ -393,13 +401,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           constexpr bool MASK = decltype(masked)::value;
           const uint64_t sl2 = pack_f32x2(p.scale_log2, p.scale_log2), nm2 = pack_f32x2(neg_ms, neg_ms);
           uint64_t acc2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
-          // the 32 scores of half c of the thread's columns, in place: the probabilities' low parts under SPLIT
+          // the 32 scores of half c of the thread's columns
           auto exp32 = [&](uint32_t (&r)[32], auto half_c) {
             constexpr int c = decltype(half_c)::value;
-            uint32_t pk[16];
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-              float p0, p1;
+            auto exp2of = [&](int e, float& p0, float& p1) {
               unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), sl2, nm2), p0, p1);
               p0 = fast_exp2(p0);
               p1 = fast_exp2(p1);
@@ -409,14 +414,38 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 p1 = (col + 1 <= c_hi && col + 1 >= c_lo) ? p1 : 0.f;
               }
               acc2[(e >> 1) & 1] = add_f32x2(acc2[(e >> 1) & 1], pack_f32x2(p0, p1));
-              pk[e / 2] = pack_bf16(p0, p1);
-              if constexpr (SPLIT) {
-                const float2 hi = unpack_bf16(pk[e / 2]);
-                r[e / 2] = pack_bf16(p0 - hi.x, p1 - hi.y);
+            };
+            if constexpr (SPLIT) {
+              // 16 scores at a time: their 24 packed words leave before the next 16 are worked on (registers)
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                uint32_t hi[8], mid[8], low[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  float p0, p1;
+                  exp2of(16 * q + 2 * i, p0, p1);
+                  hi[i] = pack_bf16(p0, p1);
+                  float2 f = unpack_bf16(hi[i]);
+                  p0 -= f.x;
+                  p1 -= f.y;
+                  mid[i] = pack_bf16(p0, p1);
+                  f = unpack_bf16(mid[i]);
+                  low[i] = pack_bf16(p0 - f.x, p1 - f.y);
+                }
+                tmem_st_x8(tP + lane_addr + half * 32 + c * 16 + q * 8, hi);
+                tmem_st_x8(tS + lane_addr + col_base + c * 32 + q * 8, mid);
+                tmem_st_x8(tS + lane_addr + col_base + c * 32 + 16 + q * 8, low);
               }
+            } else {
+              uint32_t pk[16];
+#pragma unroll
+              for (int e = 0; e < 32; e += 2) {
+                float p0, p1;
+                exp2of(e, p0, p1);
+                pk[e / 2] = pack_bf16(p0, p1);
+              }
+              tmem_st_x16(tP + lane_addr + half * 32 + c * 16, pk);
             }
-            if constexpr (SPLIT) tmem_st_x16(tS + lane_addr + col_base + c * 16, r);
-            tmem_st_x16(tP + lane_addr + half * 32 + c * 16, pk);
           };
           {
             uint32_t r[32];
@@ -428,7 +457,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
             exp32(r, IntC<0>{});
           }
-          exp32(kept, IntC<1>{});
+          if constexpr (SPLIT) {   // the parts take registers: read again (each half's parts stay in its own columns)
+            uint32_t r[32];
+            tmem_ld_x32(tS + lane_addr + col_base + 32, r);
+            tmem_ld_wait();
+            exp32(r, IntC<1>{});
+          } else {
+            exp32(kept, IntC<1>{});
+          }
           unpack_f32x2(acc2[0], sum4[0], sum4[1]);
           unpack_f32x2(acc2[1], sum4[2], sum4[3]);
         };
@@ -609,7 +645,7 @@ KWU_API int kwu_flash_fwd_mx(const void* q, int q_ld, const void* k, int k_ld, c
                         q8, sf, stream, status);
 }
 
-// As kwu_flash_fwd with probabilities carried as a bf16 pair (SPLIT above): for callers that would otherwise form
+// As kwu_flash_fwd with probabilities carried in 24 bits (SPLIT above): for callers that would otherwise form
 // attention in 32 bits.
 KWU_API int kwu_flash_fwd_split(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
                                 void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,

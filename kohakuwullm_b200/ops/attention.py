@@ -388,8 +388,8 @@ def padded_supported(q, k, v, window) -> bool:
 
 @torch.no_grad()
 def padded_attention(q, k, v, plan, window=None, sink_lse=None, scale=None):
-    """Causal attention of B rows of S tokens with probabilities that keep 16 and more mantissa bits (bf16 pairs): the
-    kernel form of ``Attention.attend`` for a prompt. q (B,S,H,64) -> (B,S,H,64)."""
+    """Causal attention of B rows of S tokens with 32-bit probabilities (three bf16 numbers each): the kernel form of
+    ``Attention.attend`` for a prompt. q (B,S,H,64) -> (B,S,H,64)."""
     L = native.require()
     B, S, H, D = q.shape
     out = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device)
