@@ -584,6 +584,10 @@ namespace kwu {
 // driver entry point fetched at run time (no link-time dependency on libcuda).
 int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_kind, uint64_t rows, uint64_t cols,
                    uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle);
+// The same of `slabs` such matrices `slab_elems` elements apart; a box lies in one slab, and what it covers past the slab's
+// last row reads as zero.
+int encode_tmap_3d(CUtensorMap* out, const void* base, int elem_kind, uint64_t slabs, uint64_t rows, uint64_t cols,
+                   uint64_t slab_elems, uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle);
 enum : int { ELEM_BF16 = 0, ELEM_F16 = 1, ELEM_U8 = 2, ELEM_F32 = 3 };
 const char* last_error();
 // Function attributes (`cudaFuncSetAttribute`) take effect per DEVICE, so "already set" is remembered per

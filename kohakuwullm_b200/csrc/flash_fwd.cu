@@ -20,7 +20,10 @@
 // softmax, which is the bound. On sums that cancel, two parts (16 bits) were 10 to 20 times as far from 64 bits as the
 // explicit fp32 form; three are nearer than it inside one key tile, and 2e-7 of the sum of magnitudes off over 3001 keys
 // (2e-8 the explicit form), where the tensor pipe's own fp32 sums are what is left. On ordinary values both forms' errors
-// are the output's bf16 rounding and agree to 1e-6. The third part costs two prompts of 3001 tokens 0.55 of 10.0 ms.
+// are the output's bf16 rounding and agree to 1e-6. The third part costs two prompts of 3001 tokens 0.55 of 10.0 ms. The rows of a padded batch are documents of one length, and
+// their tiles are loaded through maps with the row as a dimension of its own: what lies past a row's end reads as zero.
+// Read on into the next row, its values would meet probabilities of zero, and a NaN or infinity among them (0 x inf)
+// would enter the sums of this row.
 //
 // Documents never attend across their boundary: a tile's key range is clipped to its own document
 // and (with a window) to the last `window` positions. Sinks enter as sink_lse[h] = logsumexp of the
@@ -48,6 +51,7 @@ struct FlashFwdParams {
   const int4* plan;     // (q0, doc_start, doc_end, valid)
   int n_tiles;
   int T, Hq, Hkv, window;
+  int row_len;            // SPLIT: tokens of one row of the padded batch; every document is one row
   const float* sink_lse;  // (Hq) or null
   float scale_log2;       // softmax scale * log2(e)
   int* status;
@@ -187,6 +191,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tma_prefetch_desc(&tmV);
       int g = 0, ic = 0;   // K/V tiles and items issued so far by this CTA
       bool ok = true;
+      auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int token, const FwdItem& it) {
+        if constexpr (SPLIT) tma_load_3d(dst, tm, bar, col, token - it.ds, it.ds / p.row_len);
+        else tma_load_2d(dst, tm, bar, col, token);
+      };
       for (int rnd = 0; rnd * static_cast<int>(gridDim.x) < n_items && ok; ++rnd) {
         const int item = snake_item(rnd);
         if (item >= n_items) continue;
@@ -195,17 +203,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (!mbar_wait(q_empty, (ic & 1) ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_EMPTY)) break;
         ++ic;
         mbar_expect_tx(q_full, FA_TILE_BYTES);
-        tma_load_2d(sQ, &tmQ, q_full, it.h * FA_D, it.q0);
+        load(sQ, &tmQ, q_full, it.h * FA_D, it.q0, it);
         for (int j = 0; j < it.n_kv; ++j, ++g) {
           const int s = g & 1;
           const uint32_t ph = (g >> 1) & 1;
           const int kv0 = it.lo + j * FA_BN;
           if (!mbar_wait(&k_empty[s], ph ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_EMPTY)) { ok = false; break; }
           mbar_expect_tx(&k_full[s], FA_TILE_BYTES);
-          tma_load_2d(sK + s * FA_TILE_BYTES, &tmK, &k_full[s], it.hk * FA_D, kv0);
+          load(sK + s * FA_TILE_BYTES, &tmK, &k_full[s], it.hk * FA_D, kv0, it);
           if (!mbar_wait(&v_empty[s], ph ^ 1, abort_flag, p.status, KWU_ERR_TIMEOUT_EMPTY)) { ok = false; break; }
           mbar_expect_tx(&v_full[s], FA_TILE_BYTES);
-          tma_load_2d(sV + s * FA_TILE_BYTES, &tmV, &v_full[s], it.hk * FA_D, kv0);
+          load(sV + s * FA_TILE_BYTES, &tmV, &v_full[s], it.hk * FA_D, kv0, it);
         }
       }
     }
@@ -587,7 +595,7 @@ template <bool SPLIT>
 static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
                           void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
                           int window, const float* sink_lse, float scale, void* q8, void* sf, void* stream,
-                          int* status) {
+                          int* status, int row_len = 0) {
   if (T <= 0 || n_tiles <= 0) return 0;
   if (q8 && (T % 128 || (Hq * FA_D) % 128 || !sf)) {
     set_last_error("flash_fwd: the fp8 copy needs tokens and Hq * 64 in multiples of 128");
@@ -596,9 +604,17 @@ static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, cons
   if (Hq % Hkv) { set_last_error("flash_fwd: Hq must be a multiple of Hkv"); return 7; }
   CUtensorMap tmQ, tmK, tmV;
   int rc;
-  if ((rc = encode_tmap_2d(&tmQ, q, ELEM_BF16, T, (uint64_t)Hq * FA_D, q_ld, FA_BM, FA_D, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-  if ((rc = encode_tmap_2d(&tmK, k, ELEM_BF16, T, (uint64_t)Hkv * FA_D, k_ld, FA_BN, FA_D, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-  if ((rc = encode_tmap_2d(&tmV, v, ELEM_BF16, T, (uint64_t)Hkv * FA_D, v_ld, FA_BN, FA_D, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+  auto encode = [&](CUtensorMap* tm, const void* base, int heads, int ld) {
+    const uint64_t cols = static_cast<uint64_t>(heads) * FA_D;
+    if (SPLIT)
+      return encode_tmap_3d(tm, base, ELEM_BF16, T / row_len, row_len, cols, static_cast<uint64_t>(row_len) * ld, ld, FA_BM, FA_D,
+                            CU_TENSOR_MAP_SWIZZLE_128B);
+    return encode_tmap_2d(tm, base, ELEM_BF16, T, cols, ld, FA_BM, FA_D, CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  static_assert(FA_BM == FA_BN, "query and key tiles have one box");
+  if ((rc = encode(&tmQ, q, Hq, q_ld))) return rc;
+  if ((rc = encode(&tmK, k, Hkv, k_ld))) return rc;
+  if ((rc = encode(&tmV, v, Hkv, v_ld))) return rc;
   static PerDeviceOnce attr;
   if (attr.pending()) {
     cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
@@ -611,6 +627,7 @@ static int flash_fwd_impl(const void* q, int q_ld, const void* k, int k_ld, cons
   p.plan = reinterpret_cast<const int4*>(plan);
   p.n_tiles = n_tiles;
   p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.window = window;
+  p.row_len = row_len;
   p.sink_lse = sink_lse;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
@@ -645,11 +662,13 @@ KWU_API int kwu_flash_fwd_mx(const void* q, int q_ld, const void* k, int k_ld, c
                         q8, sf, stream, status);
 }
 
-// As kwu_flash_fwd with probabilities carried in 24 bits (SPLIT above): for callers that would otherwise form
-// attention in 32 bits.
+// As kwu_flash_fwd over `rows` rows of `row_len` tokens each (the documents of the plan), with probabilities carried in 24
+// bits (SPLIT above): for padded batches, whose callers would otherwise form attention in 32 bits.
 KWU_API int kwu_flash_fwd_split(const void* q, int q_ld, const void* k, int k_ld, const void* v, int v_ld,
-                                void* out, float* lse, const void* plan, int n_tiles, int T, int Hq, int Hkv,
+                                void* out, float* lse, const void* plan, int n_tiles, int rows, int row_len, int Hq, int Hkv,
                                 int window, const float* sink_lse, float scale, void* stream, int* status) {
-  return flash_fwd_impl<true>(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, T, Hq, Hkv, window, sink_lse, scale,
-                              nullptr, nullptr, stream, status);
+  if (rows <= 0 || row_len <= 0) return 0;
+  if (static_cast<long long>(rows) * row_len > 0x7fffffffLL) { set_last_error("flash_fwd_split: too many tokens"); return 7; }
+  return flash_fwd_impl<true>(q, q_ld, k, k_ld, v, v_ld, out, lse, plan, n_tiles, rows * row_len, Hq, Hkv, window, sink_lse,
+                              scale, nullptr, nullptr, stream, status, row_len);
 }

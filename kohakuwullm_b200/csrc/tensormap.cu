@@ -63,8 +63,9 @@ static EncodeTiledFn get_encode() {
   return fn;
 }
 
-int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_kind, uint64_t rows, uint64_t cols,
-                   uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle) {
+// slab_elems 0: one matrix, a map of two dimensions
+static int encode_tmap(CUtensorMap* out, const void* base, int elem_kind, uint64_t slabs, uint64_t rows, uint64_t cols,
+                       uint64_t slab_elems, uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle) {
   // The driver call needs a context bound to THIS thread (autograd runs backward on its own threads,
   // which may not have touched the runtime yet): binding the current device's primary context is cheap.
   static thread_local bool bound = false;
@@ -88,16 +89,16 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_kind, uint64_t r
     case ELEM_U8: dt = CU_TENSOR_MAP_DATA_TYPE_UINT8; eb = 1; break;
     default: dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; eb = 4; break;
   }
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld_elems * eb) & 15)) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld_elems * eb) & 15) || ((slab_elems * eb) & 15)) {
     set_last_error("TMA operand must be 16-byte aligned with a 16-byte multiple pitch (base %p pitch %llu B)",
                    base, (unsigned long long)(ld_elems * eb));
     return 2;
   }
-  cuuint64_t gdim[2] = {cols, rows};
-  cuuint64_t gstride[1] = {ld_elems * eb};
-  cuuint32_t box[2] = {box_cols, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, dt, 2, const_cast<void*>(base), gdim, gstride, box, estr,
+  cuuint64_t gdim[3] = {cols, rows, slabs};
+  cuuint64_t gstride[2] = {ld_elems * eb, slab_elems * eb};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, dt, slab_elems ? 3 : 2, const_cast<void*>(base), gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(swizzle),
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -107,6 +108,16 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_kind, uint64_t r
     return 3;
   }
   return 0;
+}
+
+int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_kind, uint64_t rows, uint64_t cols,
+                   uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle) {
+  return encode_tmap(out, base, elem_kind, 1, rows, cols, 0, ld_elems, box_rows, box_cols, swizzle);
+}
+
+int encode_tmap_3d(CUtensorMap* out, const void* base, int elem_kind, uint64_t slabs, uint64_t rows, uint64_t cols,
+                   uint64_t slab_elems, uint64_t ld_elems, uint32_t box_rows, uint32_t box_cols, int swizzle) {
+  return encode_tmap(out, base, elem_kind, slabs, rows, cols, slab_elems, ld_elems, box_rows, box_cols, swizzle);
 }
 
 }  // namespace kwu

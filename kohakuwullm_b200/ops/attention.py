@@ -396,7 +396,7 @@ def padded_attention(q, k, v, plan, window=None, sink_lse=None, scale=None):
     lse = torch.empty(H, B * S, dtype=torch.float32, device=q.device)
     rc = L.kwu_flash_fwd_split(
         native.ptr(q), c_int(q.stride(1)), native.ptr(k), c_int(k.stride(1)), native.ptr(v), c_int(v.stride(1)),
-        native.ptr(out), native.ptr(lse), native.ptr(plan), c_int(plan.shape[0] // 2), c_int(B * S), c_int(H),
+        native.ptr(out), native.ptr(lse), native.ptr(plan), c_int(plan.shape[0] // 2), c_int(B), c_int(S), c_int(H),
         c_int(k.shape[2]), c_int(window or 0), native.ptr(sink_lse), c_float(scale if scale is not None else D ** -0.5),
         native.stream_ptr(), native.ptr(native.status_word()))
     native.check(rc, "flash_fwd_split")

@@ -439,3 +439,32 @@ def test_padded_attention_keeps_32_bit_probabilities(S, spread):
     worst = ((out[0, -1].double() - want).abs() / size).max().item()
     print(f"S {S}: kernel {err:.3e} worst {worst:.3e}, explicit fp32 {base:.3e}")
     assert worst <= 2.0**-20 and err <= 2.0**-23, f"{worst} {err} (explicit form {base})"
+
+
+@pytest.mark.parametrize("S", [2, 70, 127, 129, 200])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+def test_rows_of_a_padded_batch_keep_their_values_apart(S, bad):
+    """A row's last key tile reaches over the first keys of the next row where S is no multiple of 128: what is not finite
+    there stays in its own row, and every other row is what it is without it, bit for bit."""
+    from kohakuwullm_b200.models.components.attention import Attention
+    from kohakuwullm_b200.models.seqinfo import SeqInfo
+    from kohakuwullm_b200.ops import attention as A
+    from kohakuwullm_b200.ops import native
+
+    torch.manual_seed(S)
+    B, H = 3, 2
+    q, k, v = (torch.randn(B, S, H, 64, device="cuda").bfloat16() for _ in range(3))
+    attn = Attention(64 * H, heads=H, kv_heads=H, head_dim=64).cuda()
+    info = SeqInfo.padded(B, S, device="cuda")
+    plan = A.padded_plan(info, q.device)
+    with torch.no_grad():
+        clean = A.padded_attention(q, k, v, plan, None, None, attn.scale)
+        v[1, :, 1, 5] = bad
+        k[1, 0] = bad
+        out = A.padded_attention(q, k, v, plan, None, None, attn.scale)
+        pos = info.position_ids
+        explicit = attn.attend(q, k, v, pos, pos, torch.ones(B, S, dtype=torch.bool, device="cuda"))
+    native.check_status()
+    for row in (0, 2):
+        assert torch.equal(out[row], clean[row])
+        torch.testing.assert_close(out[row].float(), explicit[row].float(), rtol=2.0**-7, atol=2.0**-9)
