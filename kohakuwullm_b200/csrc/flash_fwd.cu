@@ -118,7 +118,7 @@ __device__ __forceinline__ bool fwd_decode(const FlashFwdParams& p, int item, Fw
   it.q0 = job.x; it.ds = job.y; it.de = job.z;
   it.h = item % p.Hq;
   it.hk = it.h / (p.Hq / p.Hkv);
-  it.q_hi = min(it.q0 + FA_BM, it.de);            // one past the last valid query row
+  it.q_hi = min(min(it.q0 + FA_BM, it.de), p.T);  // one past the last valid query row; a longer plan stores nothing past T
   it.lo = it.ds;
   if (p.window > 0) it.lo = max(it.ds, it.q0 - p.window + 1);
   it.n_kv = (it.q_hi - it.lo + FA_BN - 1) / FA_BN;

@@ -105,8 +105,10 @@ class Attention(nn.Module):
         v = v.view(B, S, self.kv_heads, self.head_dim)
         q_pos = seq_info.position_ids  # (B, S) absolute positions of the queries
         # rows that count up from 0 over an empty cache (or without one) attend inside their own S columns only: packed
-        # documents of length S for the flash kernel
-        fused = plan is not None and seq_info.start is not None and (cache is None or seq_info.start == cache.length == 0) \
+        # documents of length S for the flash kernel. A layout of another shape than the tokens is left to the explicit form,
+        # which broadcasts one row of positions over the batch and refuses the rest
+        fused = isinstance(plan, attn_ops.PaddedPlan) and (plan.rows, plan.row_len) == (B, S) == tuple(q_pos.shape) \
+            and seq_info.start is not None and (cache is None or seq_info.start == cache.length == 0) \
             and getattr(self.attend, "__func__", None) is Attention.attend and not isinstance(self, SDPAAttention) \
             and attn_ops.padded_supported(q, k, v, self.window)
         if fused:

@@ -18,6 +18,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+from typing import NamedTuple
 
 import torch
 
@@ -368,14 +369,22 @@ def attention_core(qkv, q_norm, k_norm, cos, sin, cu_seqlens, plan, sink_lse, Hq
 PADDED_MAX_TILES = 2048   # the plan kernel ranks the tiles against each other in one block
 
 
-def padded_plan(seq_info, device) -> torch.Tensor | None:
+class PaddedPlan(NamedTuple):
+    """Work lists of ``rows`` documents of ``row_len`` tokens. A type of its own, so that the lists of another layout are
+    never taken for those of the tokens at hand."""
+    work: torch.Tensor
+    rows: int
+    row_len: int
+
+
+def padded_plan(seq_info, device) -> PaddedPlan | None:
     """Work lists (as :func:`attention_plan`) of a padded (B, S) batch whose rows count up from one position: B documents
     of S tokens. None when the positions are not known to do that, a row is one token (the decode kernel's case), or the
     lists would be too long."""
     B, S = seq_info.position_ids.shape
     if S < 2 or B < 1 or seq_info.start is None or B * ((S + 127) // 128) > PADDED_MAX_TILES or not native.available():
         return None
-    return attention_plan(torch.arange(0, B * S + 1, S, dtype=torch.int32, device=device), B * S)
+    return PaddedPlan(attention_plan(torch.arange(0, B * S + 1, S, dtype=torch.int32, device=device), B * S), B, S)
 
 
 def padded_supported(q, k, v, window) -> bool:
@@ -392,11 +401,13 @@ def padded_attention(q, k, v, plan, window=None, sink_lse=None, scale=None):
     ``Attention.attend`` for a prompt. q (B,S,H,64) -> (B,S,H,64)."""
     L = native.require()
     B, S, H, D = q.shape
+    if (plan.rows, plan.row_len) != (B, S) or k.shape[:2] != (B, S) or v.shape != k.shape:
+        raise ValueError(f"plan of {plan.rows} rows of {plan.row_len} tokens for q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
     out = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(H, B * S, dtype=torch.float32, device=q.device)
     rc = L.kwu_flash_fwd_split(
         native.ptr(q), c_int(q.stride(1)), native.ptr(k), c_int(k.stride(1)), native.ptr(v), c_int(v.stride(1)),
-        native.ptr(out), native.ptr(lse), native.ptr(plan), c_int(plan.shape[0] // 2), c_int(B), c_int(S), c_int(H),
+        native.ptr(out), native.ptr(lse), native.ptr(plan.work), c_int(plan.work.shape[0] // 2), c_int(B), c_int(S), c_int(H),
         c_int(k.shape[2]), c_int(window or 0), native.ptr(sink_lse), c_float(scale if scale is not None else D ** -0.5),
         native.stream_ptr(), native.ptr(native.status_word()))
     native.check(rc, "flash_fwd_split")

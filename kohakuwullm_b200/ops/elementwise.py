@@ -283,7 +283,7 @@ def qknorm_rope(x, weight, cos, sin, eps=1e-6, do_norm=True):
         _native_ok(x) and x.dim() == 3 and x.shape[-1] == 64 and x.stride(2) == 1 and x.stride(1) == 64
         and (weight is None or weight.dtype == torch.float32)
         and (cos is None or (cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-                             and cos.shape[-1] in (8, 16, 32)))
+                             and cos.shape[-1] in (8, 16, 32) and min(cos.shape[0], sin.shape[0]) >= x.shape[0]))     # the kernel reads a row a token
     )
     if ok:
         return _QKNormRope.apply(x, weight, cos, sin, eps, do_norm)

@@ -468,3 +468,28 @@ def test_rows_of_a_padded_batch_keep_their_values_apart(S, bad):
     for row in (0, 2):
         assert torch.equal(out[row], clean[row])
         torch.testing.assert_close(out[row].float(), explicit[row].float(), rtol=2.0**-7, atol=2.0**-9)
+
+
+@pytest.mark.parametrize("posenc", ["none", "rope"])
+def test_padded_calls_whose_layout_is_not_the_tokens(posenc):
+    """A layout of another shape is refused as the explicit form refuses it, and one row of positions (which the explicit
+    form broadcasts) gives what a row of positions each gives, with and without gradients."""
+    from kohakuwullm_b200.models import LMBackbone, get_preset
+    from kohakuwullm_b200.models.seqinfo import SeqInfo
+    from kohakuwullm_b200.ops import native
+
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        model = LMBackbone(get_preset("B200-smoke", vocab_size=512, posenc=posenc)).to(torch.bfloat16).eval()
+    B, S = 3, 130
+    ids = torch.randint(0, 512, (B, S), device="cuda")
+    with torch.no_grad():
+        want = model(ids, SeqInfo.padded(B, S, device="cuda"))
+        for layout in ((B, S + 1), (B, S - 1), (B - 1, S)):
+            with pytest.raises(RuntimeError):
+                model(ids, SeqInfo.padded(*layout, device="cuda"))
+        if posenc == "none":
+            one = model(ids, SeqInfo.padded(1, S, device="cuda"))
+            torch.testing.assert_close(one.float(), want.float(), rtol=5e-2, atol=5e-2)
+    torch.cuda.synchronize()
+    native.check_status()

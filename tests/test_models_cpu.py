@@ -149,3 +149,68 @@ def test_nd_rotary_encodings_rotate_by_position_vectors():
     assert torch.allclose(torch.cos(ang(3)), torch.cos(want), atol=1e-5)
     learn = GGRoPE(head_dim=32, position_dim=2)
     assert any(p.requires_grad for p in learn.parameters())
+
+
+@pytest.mark.parametrize("rows,cols,layout,fused", [(3, 7, (3, 7), True), (3, 7, (1, 7), False), (3, 7, (3, 8), False),
+                                                    (3, 7, (3, 6), False), (3, 7, (2, 7), False), (3, 8, (4, 6), False)])
+@pytest.mark.parametrize("plan_of", ["layout", "tokens"])
+def test_padded_kernel_runs_only_on_a_layout_of_the_tokens_shape(monkeypatch, rows, cols, layout, fused, plan_of):
+    """The kernel takes its rows from the plan and its buffers from the tokens, so it runs only where both agree with the
+    positions. One row of positions broadcasts over the batch in the explicit form; other shapes are refused by it."""
+    from kohakuwullm_b200.models.components.attention import Attention
+    from kohakuwullm_b200.ops import attention as A
+
+    torch.manual_seed(0)
+    attn = Attention(64, heads=2, kv_heads=1, head_dim=32, qk_norm=False)
+    for w in attn.parameters():
+        torch.nn.init.normal_(w, std=0.1)
+    x = torch.randn(rows, cols, 64)
+    ran = []
+
+    def kernel(q, k, v, plan, *a):
+        ran.append((plan.rows, plan.row_len))
+        return torch.zeros_like(q)
+
+    monkeypatch.setattr(A, "padded_supported", lambda *a: True)
+    monkeypatch.setattr(A, "padded_attention", kernel)
+    info = SeqInfo.padded(*layout)
+    plan = A.PaddedPlan(torch.zeros(0, 4), *(layout if plan_of == "layout" else (rows, cols)))
+    with torch.no_grad():
+        if layout == (1, cols):
+            want = attn(x, SeqInfo.padded(rows, cols))
+            assert torch.equal(attn(x, info, plan=plan), want)
+        elif not fused:
+            with pytest.raises(RuntimeError):
+                attn(x, info, plan=plan)
+        else:
+            attn(x, info, plan=plan)
+        assert ran == ([(rows, cols)] if fused else [])
+        ran.clear()
+        attn(x, SeqInfo.padded(rows, cols), plan=torch.zeros(4, 4))       # the lists of a packed layout
+        assert not ran
+
+
+def test_padded_attention_refuses_the_plan_of_another_shape(monkeypatch):
+    from kohakuwullm_b200.ops import attention as A
+
+    monkeypatch.setattr(A.native, "require", lambda: None)
+    q = torch.zeros(2, 7, 2, 64)
+    for rows, row_len in ((2, 8), (3, 7), (1, 14), (14, 1)):
+        with pytest.raises(ValueError, match="plan of"):
+            A.padded_attention(q, q, q, A.PaddedPlan(torch.zeros(2, 4), rows, row_len))
+    with pytest.raises(ValueError, match="plan of"):
+        A.padded_attention(q, q[:, :3], q[:, :3], A.PaddedPlan(torch.zeros(2, 4), 2, 7))
+
+
+def test_rotary_tables_shorter_than_the_tokens_never_reach_the_kernel(monkeypatch):
+    from kohakuwullm_b200.ops import elementwise as E
+
+    monkeypatch.setattr(E, "_native_ok", lambda *a: True)
+    monkeypatch.setattr(E._QKNormRope, "apply", lambda *a: "kernel")
+    x = torch.randn(10, 2, 64)
+    for n in (10, 12):
+        ang = torch.rand(n, 32)
+        assert E.qknorm_rope(x, None, ang.cos(), ang.sin()) == "kernel"
+    ang = torch.rand(9, 32)
+    with pytest.raises(RuntimeError):
+        E.qknorm_rope(x, None, ang.cos(), ang.sin())
