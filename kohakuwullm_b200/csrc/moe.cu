@@ -15,6 +15,8 @@
 #include "common.cuh"
 #include "mx_quant.cuh"
 
+#include <cfloat>
+
 namespace kwu {
 
 constexpr int RT_BT = 32;     // tokens per block
@@ -108,7 +110,11 @@ moe_router_fwd_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float*
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int e = lane + 32 * j;
-      sel[j] = e < E ? sc[j] + (bias ? bias[e] : 0.f) : -INFINITY;
+      // Every expert stays above -inf, which marks lanes without an expert and experts already picked: a token whose scores
+      // are NaN (a diverged step) still gets top_k different experts, on which the placement and the combine index memory.
+      // The NaN goes on in its gate weights.
+      const float s = e < E ? sc[j] + (bias ? bias[e] : 0.f) : -INFINITY;
+      sel[j] = e < E && !(s >= -FLT_MAX) ? -FLT_MAX : s;
     }
     float wsum = 0.f;
     float my_w = 0.f;
@@ -187,7 +193,8 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int E, int* __re
 
 // A block ranks its pairs inside each expert in shared memory and takes one range of the expert's rows for all of them.
 // One returning addition per pair on the few cursors of the experts serialised in the L2: 23.4 us for 49152 pairs over
-// 64 experts, below 10 like this (the router's picks counted the same way: 27.3 and 13.9 us).
+// 64 experts, below 10 like this (the router's picks counted the same way: 27.3 and 13.9 us). A pair whose id is no expert
+// takes no row (its position is row 0, so that what gathers by position stays inside the buffer).
 constexpr int MOE_PLACE_THREADS = 512;
 __global__ void __launch_bounds__(MOE_PLACE_THREADS)
 moe_place_kernel(const int* __restrict__ idx, int n_pairs, const int* __restrict__ offsets, int* __restrict__ cursors,
@@ -196,16 +203,17 @@ moe_place_kernel(const int* __restrict__ idx, int n_pairs, const int* __restrict
   for (int e = threadIdx.x; e < E; e += blockDim.x) s_n[e] = 0;
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int e = i < n_pairs ? idx[i] : 0;
-  const int rank = i < n_pairs ? atomicAdd(&s_n[e], 1) : 0;
+  const int e = i < n_pairs ? idx[i] : -1;
+  const bool known = static_cast<unsigned>(e) < static_cast<unsigned>(E);
+  const int rank = known ? atomicAdd(&s_n[e], 1) : 0;
   __syncthreads();
   for (int x = threadIdx.x; x < E; x += blockDim.x)
     if (s_n[x]) s_base[x] = offsets[x] + atomicAdd(&cursors[x], s_n[x]);
   __syncthreads();
   if (i >= n_pairs) return;
-  const int pos = s_base[e] + rank;
+  const int pos = known ? s_base[e] + rank : 0;
   pos_of[i] = pos;
-  pair_of[pos] = i;
+  if (known) pair_of[pos] = i;
 }
 
 // rows[pos] = x[pair_of[pos] / k] (zero when the row is padding). One warp per row. With `mx` the MXFP8 copy of

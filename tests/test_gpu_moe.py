@@ -177,3 +177,65 @@ def test_router_backward_matches_eager(score, norm_topk):
     # the products run on the tensor cores with a bf16 copy of the logit gradient: bf16-level agreement
     torch.testing.assert_close(dW_n, dW_e, rtol=2e-2, atol=1e-2 * dW_e.abs().max().item())
     torch.testing.assert_close(dx_n, dx_e, rtol=2e-2, atol=2e-2 * dx_e.abs().max().item())
+
+
+@pytest.mark.parametrize("E,k", [(8, 8), (24, 4), (64, 6), (128, 8)])
+@pytest.mark.parametrize("score", ["sigmoid", "softmax", "sqrtsoftplus"])
+def test_tokens_without_finite_scores_get_experts_that_exist(E, k, score):
+    """Rows of NaN, of one infinite input (scores of inf and NaN) and, with masked experts, of -inf among ordinary ones:
+    every token gets k different ids in [0, E), the counts hold T k picks, ordinary tokens are routed as without them."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.moe import router_topk
+
+    torch.manual_seed(E + k)
+    T, D = 70, 256
+    W = torch.randn(E, D, device="cuda") * 0.5
+    bias = torch.randn(E, device="cuda")
+    if k < E:
+        bias[E - (E - k) // 2 - 1:] = float("-inf")     # never picked while others are left
+    x = torch.randn(T, D, device="cuda", dtype=torch.bfloat16)
+    clean = router_topk(x, W, bias, None, k, score)
+    bad = torch.tensor([0, 31, 32, 69], device="cuda")
+    x[bad] = float("nan")
+    x[5, 7] = float("inf")
+    load = torch.zeros(E, device="cuda")
+    idx, weight, counts, _ = router_topk(x, W, bias, load, k, score)
+    torch.cuda.synchronize()
+    native.check_status()
+    assert ((idx >= 0) & (idx < E)).all()
+    assert (idx.sort(-1).values.diff(dim=-1) > 0).all()
+    assert torch.equal(counts.long(), torch.bincount(idx.reshape(-1).long(), minlength=E)) and counts.sum() == T * k
+    assert torch.equal(load, counts.float())
+    assert weight[bad].isnan().all()
+    rest = torch.ones(T, dtype=torch.bool, device="cuda")
+    rest[bad] = rest[5] = False
+    assert torch.equal(idx[rest], clean[0][rest]) and torch.equal(weight[rest], clean[1][rest])
+
+
+@pytest.mark.parametrize("E", [8, 128])
+def test_placement_leaves_out_ids_that_are_no_expert(E):
+    """Pairs of an id outside [0, E) take no row; the others fill their experts' rows, and every position is inside."""
+    import ctypes
+
+    from kohakuwullm_b200.ops import native
+
+    torch.manual_seed(E)
+    n = 1300
+    idx = torch.randint(0, E, (n,), device="cuda", dtype=torch.int32)
+    odd = torch.tensor([0, 511, 512, 1299], device="cuda")
+    idx[odd] = torch.tensor([E, -1, E + 5, 1 << 20], device="cuda", dtype=torch.int32)
+    valid = torch.ones(n, dtype=torch.bool, device="cuda")
+    valid[odd] = False
+    counts = torch.bincount(idx[valid].long(), minlength=E).to(torch.int32)
+    L, ci = native.require(), ctypes.c_int
+    rows = L.kwu_moe_max_rows(ci(n), ci(E))
+    new = lambda *shape: torch.full(shape, -7, dtype=torch.int32, device="cuda")
+    offsets, cursors, tiles, pos, pair = new(E + 1), new(E), new(rows // 128, 4), new(n), new(rows)
+    native.check(L.kwu_moe_plan_and_place(native.ptr(counts), native.ptr(idx), ci(n), ci(E), native.ptr(offsets),
+                                          native.ptr(cursors), native.ptr(tiles), ci(rows // 128), native.ptr(pos),
+                                          native.ptr(pair), ci(rows), native.stream_ptr()), "place")
+    assert ((pos >= 0) & (pos < rows)).all() and (pos[odd] == 0).all()
+    e = idx[valid].long()
+    assert (pos[valid] >= offsets[e]).all() and (pos[valid] < offsets[e] + counts[e]).all()
+    assert torch.equal(pair[pos[valid].long()].long(), torch.nonzero(valid).flatten())
+    assert (pair >= 0).sum() == valid.sum()
