@@ -13,8 +13,9 @@ from dataclasses import dataclass, field, replace
 import torch
 
 
-def _version(t: torch.Tensor) -> int:
-    return -1 if t.is_inference() else t._version
+def _version(t: torch.Tensor) -> int | None:
+    """Count of the writes into ``t``; None for inference tensors, which have no such count."""
+    return None if t.is_inference() else t._version
 
 
 @dataclass
@@ -26,7 +27,7 @@ class SeqInfo:
     # host copy of the document lengths (kept so FLOP accounting and splitters never sync)
     lengths: tuple[int, ...] | None = None
     # (first position, version of ``position_ids``) when every row is known to count up from one host-known position
-    _count: tuple[int, int] | None = field(default=None, init=False, repr=False, compare=False)
+    _count: tuple[int, int | None] | None = field(default=None, init=False, repr=False, compare=False)
 
     def __setattr__(self, name, value):
         if name == "position_ids":
@@ -36,10 +37,20 @@ class SeqInfo:
     @property
     def start(self) -> int | None:
         """Position of the first column when every row of a padded batch is ``start, start + 1, ...``, known without
-        reading the device; None when the positions were given, replaced or written to."""
-        if self._count is None or _version(self.position_ids) != self._count[1]:
+        reading the device; None when the positions were given, replaced or written to, or are an inference tensor (whose
+        writes torch does not count)."""
+        if self._count is None or self._count[1] is None or _version(self.position_ids) != self._count[1]:
             return None
         return self._count[0]
+
+    # a copied or unpickled tensor counts its writes anew, so what is known goes over as the bare position
+    def __getstate__(self):
+        return {**self.__dict__, "_count": self.start}
+
+    def __setstate__(self, state):
+        start = state.get("_count")
+        self.__dict__.update(state)
+        self._count = None if start is None else (start, _version(self.position_ids))
 
     @property
     def packed(self) -> bool:

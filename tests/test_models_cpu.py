@@ -214,3 +214,31 @@ def test_rotary_tables_shorter_than_the_tokens_never_reach_the_kernel(monkeypatc
     ang = torch.rand(9, 32)
     with pytest.raises(RuntimeError):
         E.qknorm_rope(x, None, ang.cos(), ang.sin())
+
+
+def test_known_positions_are_forgotten_with_every_write():
+    """``SeqInfo.start`` lets a kernel leave out the positions, so it is known only while nothing has written to them: not
+    for inference tensors (torch counts no writes there) and not in a copy made after a write, whose count starts anew."""
+    import copy
+    import pickle
+
+    with torch.inference_mode():
+        info = SeqInfo.padded(2, 5, offset=1)
+        assert info.start is None
+        info.position_ids.add_(3)
+        assert info.start is None
+        plain = SeqInfo.padded(1, 5).to("cpu")
+        assert plain.start is None
+    kept = SeqInfo.padded(1, 5, offset=4)
+    with torch.inference_mode():
+        assert kept.start == 4
+        kept.position_ids[0, 2] = 9
+        assert kept.start is None
+    for clone in (copy.copy, copy.deepcopy, lambda t: pickle.loads(pickle.dumps(t))):
+        info = SeqInfo.padded(1, 5, offset=2)
+        other = clone(info)
+        assert other.start == 2 and torch.equal(other.position_ids, info.position_ids)
+        other.position_ids.add_(1)
+        assert other.start is None and (info.start is None) == (clone is copy.copy)
+        info.position_ids.add_(1)
+        assert info.start is None and clone(info).start is None and clone(info) is not info
