@@ -39,9 +39,13 @@ class KVCache:
     def append(self, layer: int, k: torch.Tensor, v: torch.Tensor, q_pos: torch.Tensor):
         """Store this step's keys/values; returns ``(k_all, v_all, key_positions, key_valid)``."""
         k_all, v_all = self.store(layer, k, v)
+        return k_all, v_all, *self.key_positions(k_all, k.shape[1])
+
+    def key_positions(self, k_all: torch.Tensor, new: int):
+        """Positions of the keys in ``k_all`` and which of them exist, once ``new`` ones are stored."""
         B, used = k_all.shape[:2]
-        pos = torch.arange(used, device=k.device)[None, :].expand(B, used)
-        return k_all, v_all, pos, pos < self.length + k.shape[1]
+        pos = torch.arange(used, device=k_all.device)[None, :].expand(B, used)
+        return pos, pos < self.length + new
 
     def store(self, layer: int, k: torch.Tensor, v: torch.Tensor):
         """:meth:`append` for kernels that know which keys exist: returns ``(k_all, v_all)`` alone."""
@@ -80,3 +84,18 @@ class KVCache:
     def reset(self) -> None:
         self.length = 0
         self._pending = 0
+        self.position = None
+
+
+_APPEND = KVCache.append
+
+
+def stores_plainly(cache) -> bool:
+    """Whether ``cache`` keeps keys and values the way :meth:`KVCache.append` does, so that a kernel may go without the
+    positions that it returns. A cache with an ``append`` of its own is asked through it."""
+    return getattr(getattr(cache, "append", None), "__func__", None) is _APPEND
+
+
+def keeps_as_is(buffer: torch.Tensor | None, x: torch.Tensor) -> bool:
+    """Whether storing ``x`` (B, S, ...) changes nothing about it: a new buffer, or one of its type and batch size."""
+    return buffer is None or (buffer.dtype == x.dtype and buffer.shape[0] == x.shape[0])

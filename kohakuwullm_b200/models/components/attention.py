@@ -22,6 +22,7 @@ import math
 import torch
 from torch import nn
 
+from kohakuwullm_b200.models.cache import keeps_as_is, stores_plainly
 from kohakuwullm_b200.models.components.mlp import Linear
 from kohakuwullm_b200.ops import attention as attn_ops
 from kohakuwullm_b200.ops.attention import varlen_attention
@@ -107,8 +108,11 @@ class Attention(nn.Module):
         # rows that count up from 0 over an empty cache (or without one) attend inside their own S columns only: packed
         # documents of length S for the flash kernel. A layout of another shape than the tokens is left to the explicit form,
         # which broadcasts one row of positions over the batch and refuses the rest
+        plain = cache is None or stores_plainly(cache)
         fused = isinstance(plan, attn_ops.PaddedPlan) and (plan.rows, plan.row_len) == (B, S) == tuple(q_pos.shape) \
-            and seq_info.start is not None and (cache is None or seq_info.start == cache.length == 0) \
+            and seq_info.start is not None and plain \
+            and (cache is None or (seq_info.start == cache.length == 0 and keeps_as_is(cache.k[layer], k)
+                                   and keeps_as_is(cache.v[layer], v))) \
             and getattr(self.attend, "__func__", None) is Attention.attend and not isinstance(self, SDPAAttention) \
             and attn_ops.padded_supported(q, k, v, self.window)
         if fused:
@@ -118,17 +122,18 @@ class Attention(nn.Module):
             return self.o_proj(out.reshape(B, S, self.q_dim))
         if cache is not None:
             # the decode kernel needs no key positions
-            decode = S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) and q.is_contiguous()
-            if decode:
+            if plain:
                 k, v = cache.store(layer, k, v)
             else:
                 k, v, k_pos, k_valid = cache.append(layer, k, v, q_pos)
-            if decode:
+            if S == 1 and not torch.is_grad_enabled() and attn_ops.decode_supported(q[:, 0], k) and q.is_contiguous():
                 # one new token per row: split-KV decode kernel straight over the cache buffers
-                held = cache.position is not None
+                held = plain and cache.position is not None
                 out = attn_ops.decode_attention(q[:, 0], k, v, k.shape[1] if held else cache.length + 1, self.window,
                                                 self.scale, self.sink, position=cache.position[1] if held else None)
                 return self.o_proj(out.reshape(B, 1, self.q_dim))
+            if plain:
+                k_pos, k_valid = cache.key_positions(k, S)
         else:
             k_pos = q_pos
             k_valid = torch.ones(B, S, dtype=torch.bool, device=x.device)

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import kohakuwullm_b200.models  # noqa: F401  (the import that must register every built-in component)
-from kohakuwullm_b200.models import LMBackbone, get_preset
+from kohakuwullm_b200.models import KVCache, LMBackbone, get_preset
 from kohakuwullm_b200.models.seqinfo import SeqInfo
 from kohakuwullm_b200.registry import ATTENTION, MLP, NORM, POSENC, ROUTER
 
@@ -242,3 +242,95 @@ def test_known_positions_are_forgotten_with_every_write():
         assert other.start is None and (info.start is None) == (clone is copy.copy)
         info.position_ids.add_(1)
         assert info.start is None and clone(info).start is None and clone(info) is not info
+
+
+class _Rounding(KVCache):
+    """A cache with an ``append`` of its own: keeps its keys and values in a narrower type."""
+
+    def append(self, layer, k, v, q_pos):
+        self.seen = getattr(self, "seen", 0) + 1
+        return super().append(layer, (k * 8).round() / 8, v, q_pos)
+
+
+class _Foreign:
+    """A cache that is no KVCache and has nothing but what the backbone asks of one."""
+
+    def __init__(self, depth, max_len):
+        self.inner, self.seen = KVCache(depth, max_len, static=False), 0
+
+    length = property(lambda self: self.inner.length)
+
+    def append(self, *args):
+        self.seen += 1
+        return self.inner.append(*args)
+
+    def advance(self):
+        self.inner.advance()
+
+
+@pytest.mark.parametrize("kind", ["subclass", "instance", "foreign", "plain"])
+def test_a_cache_with_its_own_append_is_asked_through_it(monkeypatch, kind):
+    """Prompt and decode go through ``append`` where a cache brings its own, kernels or not."""
+    from kohakuwullm_b200.ops import attention as A
+
+    torch.manual_seed(0)
+    cfg = get_preset("B200-smoke", **BASE)
+    model = LMBackbone(cfg).eval()
+    tokens = torch.randint(0, 128, (2, 6))
+    kernels = []
+    monkeypatch.setattr(A, "padded_plan", lambda info, device: A.PaddedPlan(torch.zeros(0, 4), *info.position_ids.shape))
+    monkeypatch.setattr(LMBackbone, "prepare", lambda self, info, device, dtype: (
+        self.pos_enc.prepare(info.position_ids), A.padded_plan(info, device)))
+    monkeypatch.setattr(A, "padded_supported", lambda *a: True)
+    monkeypatch.setattr(A, "padded_attention", lambda q, *a: kernels.append("prompt") or torch.zeros_like(q))
+    monkeypatch.setattr(A, "decode_supported", lambda *a: True)
+    monkeypatch.setattr(A, "decode_attention", lambda q, *a, **k: kernels.append("decode") or torch.zeros_like(q))
+    cache = {"subclass": _Rounding, "foreign": _Foreign}.get(kind, KVCache)(cfg.depth, 16)
+    if kind == "instance":
+        cache.seen = 0
+        cache.append = lambda *a: (setattr(cache, "seen", cache.seen + 1), KVCache.append(cache, *a))[1]
+    with torch.no_grad():
+        info = SeqInfo.padded(2, 6)
+        model(tokens, info, cache=cache)
+        model(tokens[:, :1], SeqInfo.padded(2, 1, offset=6), cache=cache)
+    assert cache.length == 7
+    if kind == "plain":
+        assert kernels == ["prompt", "prompt", "decode", "decode"]
+    else:
+        assert kernels == ["decode", "decode"] and cache.seen == 4
+
+
+def test_kernels_read_only_cache_buffers_of_the_keys_own_type(monkeypatch):
+    """A cache whose buffers are wider than the model's keys holds rounded or widened copies: prompt and decode attend over
+    what it holds, in the explicit form."""
+    from kohakuwullm_b200.ops import attention as A
+
+    torch.manual_seed(0)
+    cfg = get_preset("B200-smoke", **BASE)
+    model = LMBackbone(cfg).eval()
+    tokens = torch.randint(0, 128, (2, 6))
+    monkeypatch.setattr(LMBackbone, "prepare", lambda self, info, device, dtype: (
+        self.pos_enc.prepare(info.position_ids), A.PaddedPlan(torch.zeros(0, 4), *info.position_ids.shape)))
+    monkeypatch.setattr(A, "padded_supported", lambda *a: True)
+    monkeypatch.setattr(A, "padded_attention", lambda *a: pytest.fail("prompt kernel over a buffer of another type"))
+    monkeypatch.setattr(A, "decode_supported", lambda q, k: k.dtype == torch.float32)
+    monkeypatch.setattr(A, "decode_attention", lambda *a, **k: pytest.fail("decode kernel over a buffer of another type"))
+    cache, want = KVCache(cfg.depth, 16), KVCache(cfg.depth, 16, static=False)
+    shape = (2, 16, cfg.kv_heads, cfg.head_dim)
+    cache.k = [torch.zeros(shape, dtype=torch.float64) for _ in range(cfg.depth)]
+    cache.v = [torch.zeros(shape, dtype=torch.float64) for _ in range(cfg.depth)]
+    with torch.no_grad():
+        got = [model(tokens, SeqInfo.padded(2, 6), cache=cache), model(tokens[:, :1], SeqInfo.padded(2, 1, offset=6), cache=cache)]
+    with torch.enable_grad():     # no kernel
+        monkeypatch.setattr(A, "padded_supported", lambda *a: False)
+        ref = [model(tokens, SeqInfo.padded(2, 6), cache=want), model(tokens[:, :1], SeqInfo.padded(2, 1, offset=6), cache=want)]
+    for a, b in zip(got, ref):
+        torch.testing.assert_close(a, b.detach(), rtol=1e-5, atol=1e-5)
+
+
+def test_a_reset_cache_holds_no_device_position():
+    cache = KVCache(2, 16)
+    cache.length = 5
+    cache.hold_position("cpu")
+    cache.reset()
+    assert cache.position is None and cache.seq_info(torch.zeros(1, 3)).start == 0
