@@ -16,6 +16,7 @@ Reference: src/kohakuwullm/generation/engine.py:19-385.
 
 from __future__ import annotations
 
+import warnings
 from typing import Sequence
 
 import torch
@@ -129,8 +130,8 @@ class StepGraph:
 
 def capturable(backbone, tokens: torch.Tensor) -> bool:
     """Whether a cached one-token step of this model is a fixed sequence of kernels: every module is one whose decode path
-    reads nothing back to the host, runs on the native kernels, and carries no hooks or replaced methods that a replay
-    would skip."""
+    reads nothing back to the host, runs on the native kernels, and carries no hooks, modes or replaced methods that a
+    replay would skip."""
     from torch.nn.modules import module as hooks
 
     from kohakuwullm_b200.models.backbone import LMBackbone
@@ -144,6 +145,9 @@ def capturable(backbone, tokens: torch.Tensor) -> bool:
              torch.nn.Identity)
     if type(backbone) is not LMBackbone or not tokens.is_cuda or not native.available() \
             or torch.cuda.is_current_stream_capturing() or hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
+        return False
+    # dispatch and function modes (operation counters, loggers) see every operator of a step issued directly
+    if torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack():
         return False
     if backbone.embed.weight.dtype != torch.bfloat16 or backbone.config.head_dim != 64:
         return False
@@ -202,7 +206,8 @@ class LocalGenerator:
             if graphs and graph is None and i >= 2 and max_new_tokens - i >= StepGraph.MIN_STEPS:
                 try:
                     graph = StepGraph(bb, cache, step_in, self._captures.pop(str(prompt.device), None))
-                except RuntimeError:       # what cannot be captured is issued directly, and raises there if it is wrong
+                except RuntimeError as err:    # what cannot be captured is issued directly, and raises there if it is wrong
+                    warnings.warn(f"decode steps are issued one by one, their capture failed: {err}")
                     graphs = False
             if graph is not None:
                 logits = graph(cache, step_in)

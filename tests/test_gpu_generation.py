@@ -24,7 +24,8 @@ def _model(**kw):
 @pytest.mark.parametrize("kw,rows,prompt,new", [
     ({}, 1, 5, 9), ({}, 3, 250, 14),                                      # the cache crosses a chunk of 256 keys
     (dict(sliding_window=16, global_layer_every=2, attn_sink=True, attn_num_sinks=2), 2, 10, 24),
-    (dict(sliding_window=300), 2, 290, 20), (dict(preset="Kohaku-MoE-1B", depth=3), 2, 20, 8)])
+    (dict(sliding_window=300), 2, 290, 20), (dict(preset="Kohaku-MoE-1B", depth=3), 2, 20, 8),
+    (dict(preset="B200-dense-546M", depth=3, mxfp8=True), 3, 20, 8), (dict(preset="Kohaku-MoE-1B", depth=3, mxfp8=True), 2, 20, 8)])
 def test_captured_steps_give_the_tokens_of_direct_steps(kw, rows, prompt, new):
     from kohakuwullm_b200.generation.engine import LocalGenerator, StepGraph, capturable
     from kohakuwullm_b200.ops import native
@@ -68,3 +69,40 @@ def test_models_that_read_back_or_are_altered_are_not_captured():
     model.head.logits = lambda h: h
     assert not capturable(model, tokens)
     assert not capturable(_model().float(), tokens)
+
+
+def test_modes_see_every_decode_step():
+    """A dispatch or function mode (an operation counter) around a call sees all of its steps: none is replayed."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from kohakuwullm_b200.generation.engine import LocalGenerator, capturable
+
+    class Dispatch(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen += 1
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        seen = 0
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.seen += 1
+            return func(*args, **(kwargs or {}))
+
+    model = _model()
+    tokens = torch.randint(1, 512, (1, 5), device="cuda")
+    gen = LocalGenerator(model, eos_id=511, stop_ids=(600,))
+    want = gen.generate(tokens, 24, temperature=0.0)
+    for mode in (Dispatch, Function):
+        counts = []
+        for new in (8, 16, 24):
+            with mode() as m:
+                assert not capturable(model, tokens)
+                got = gen.generate(tokens, new, temperature=0.0)
+            counts.append(m.seen)
+        assert torch.equal(got, want)
+        assert counts[2] - counts[1] == counts[1] - counts[0] > 8 * model.config.depth    # the same for each eight steps
+    assert capturable(model, tokens)
