@@ -16,6 +16,7 @@ Reference: src/kohakuwullm/generation/engine.py:19-385.
 
 from __future__ import annotations
 
+import ctypes
 import warnings
 from typing import Sequence
 
@@ -24,6 +25,8 @@ import torch.distributed as dist
 
 from kohakuwullm_b200.models.cache import KVCache
 from kohakuwullm_b200.models.seqinfo import SeqInfo
+from kohakuwullm_b200.ops import native
+from kohakuwullm_b200.ops.mxfp8 import clear_prequantized
 
 SAMPLE_SEED = 20090220
 
@@ -86,46 +89,69 @@ def advance(tokens: torch.Tensor, nxt: torch.Tensor, finished: torch.Tensor, sto
     return torch.cat([tokens, nxt[:, None]], dim=1), finished | hit
 
 
+class CapturePool:
+    """Memory and stream of captured steps, one capture at a time: the next one takes over what the last one has left."""
+
+    def __init__(self, device):
+        self.lib, handle = native.require(), ctypes.c_void_p()
+        with torch.cuda.device(device):
+            self.memory = torch.cuda.MemPool()
+            native.check(self.lib.kwu_stream_create(ctypes.byref(handle)), "stream of decode captures")
+        # blocks of the memory belong to the stream that they were made on
+        self.stream = torch.cuda.ExternalStream(handle.value, device=device)
+
+    def __del__(self):
+        if getattr(self, "stream", None) is not None:
+            self.lib.kwu_stream_destroy(ctypes.c_void_p(self.stream.cuda_stream))
+
+
 class StepGraph:
     """One cached decode step (embedding to logits of one new token a row) captured as a CUDA graph.
 
     A step is 15 to 20 short kernels a layer; issued from Python they leave the GPU idle for most of the step, replayed
     they follow each other. The position lives on the device (``KVCache.hold_position``), so one capture serves every
-    remaining token of the call. ``earlier``: a finished capture whose memory this one takes over."""
+    remaining token of the call. The capture is the library's own and not torch's, whose captures make every other thread's
+    draw from the device's default generator fail for as long as they last."""
 
     MIN_STEPS = 3     # a capture costs about a step issued from Python, so it pays from the third on
 
-    def __init__(self, backbone, cache, token: torch.Tensor, earlier: "StepGraph | None" = None):
+    def __init__(self, backbone, cache, token: torch.Tensor, pool: CapturePool):
+        self.lib, self.exec = native.require(), ctypes.c_void_p()
         self.token = token.clone()
-        self.graph = torch.cuda.CUDAGraph()
         length = cache.length
         cache.hold_position(token.device)
-        # the memory of a capture belongs to its stream: the next capture can take it over only there
-        self.stream = stream = torch.cuda.Stream(device=token.device) if earlier is None else earlier.stream
-        stream.wait_stream(torch.cuda.current_stream(token.device))
+        handle = ctypes.c_void_p(pool.stream.cuda_stream)
+        pool.stream.wait_stream(torch.cuda.current_stream(token.device))
         try:
-            with torch.cuda.stream(stream):
-                # thread-local: other threads of the program may go on allocating and synchronising
-                pool = () if earlier is None else (earlier.graph.pool(),)
-                self.graph.capture_begin(*pool, capture_error_mode="thread_local")
+            with torch.cuda.stream(pool.stream), torch.cuda.use_mem_pool(pool.memory, token.device):
+                native.check(self.lib.kwu_capture_begin(handle), "capture of a decode step")
+                exec_at = None
                 try:
                     hidden = backbone(self.token, cache.seq_info(self.token), cache=cache)
                     self.logits = backbone.head.logits(hidden[:, -1])
+                    exec_at = ctypes.byref(self.exec)
                 finally:
-                    self.graph.capture_end()
+                    rc = self.lib.kwu_capture_end(handle, exec_at)     # also ends a capture that failed on the way
+                native.check(rc, "capture of a decode step")
         except BaseException:
             cache.position = None
             raise
         finally:
             cache.length, cache._pending = length, 0      # nothing has run yet
+            if backbone.config.mxfp8:
+                clear_prequantized()                       # copies that the capture has made and nothing took
 
     def __call__(self, cache, token: torch.Tensor) -> torch.Tensor:
         if cache.length + 1 > cache.max_len:
             raise RuntimeError(f"KV cache overflow: {cache.length + 1} > max_len {cache.max_len}")
         self.token.copy_(token)
-        self.graph.replay()
+        native.check(self.lib.kwu_graph_launch(self.exec, native.stream_ptr()), "decode step")
         cache.length += 1
         return self.logits
+
+    def __del__(self):
+        if getattr(self, "exec", None):
+            self.lib.kwu_graph_destroy(self.exec)
 
 
 def capturable(backbone, tokens: torch.Tensor) -> bool:
@@ -138,7 +164,6 @@ def capturable(backbone, tokens: torch.Tensor) -> bool:
     from kohakuwullm_b200.models.block import DecoderBlock
     from kohakuwullm_b200.models.components import attention, mlp, moe, norm, posenc
     from kohakuwullm_b200.models.head import LMHead
-    from kohakuwullm_b200.ops import native
 
     plain = (LMBackbone, DecoderBlock, LMHead, mlp.Linear, mlp.GLUMLP, mlp.GeGLUMLP, mlp.GELUMLP, norm.RMSNorm,
              norm.GemmaRMSNorm, norm.LayerNorm, norm.DyT, posenc.RoPE, posenc.NoPE, torch.nn.Embedding, torch.nn.ModuleList,
@@ -178,7 +203,7 @@ class LocalGenerator:
         self.stop_ids = tuple(stop_ids) or (eos_id,)
         self.use_cache, self.static_cache = use_cache, static_cache
         self._rng: dict[str, torch.Generator] = {}
-        self._captures: dict[str, StepGraph] = {}     # the last finished capture of a device, for its memory
+        self._pools: dict[str, CapturePool] = {}      # what the last finished call on a device captured into
 
     def rng(self, device) -> torch.Generator:
         key = str(device)
@@ -200,12 +225,14 @@ class LocalGenerator:
         gen = self.rng(prompt.device)
         cache = KVCache.from_config(bb.config, S + max_new_tokens, static=self.static_cache) if self.use_cache else None
         step_in = prompt
-        graph, graphs = None, cache is not None and self.static_cache and capturable(bb, prompt)
+        graph, pool, graphs = None, None, cache is not None and self.static_cache and capturable(bb, prompt)
         for i in range(max_new_tokens):
             # the first one-token step is issued directly: it loads kernels and builds what later ones find
             if graphs and graph is None and i >= 2 and max_new_tokens - i >= StepGraph.MIN_STEPS:
                 try:
-                    graph = StepGraph(bb, cache, step_in, self._captures.pop(str(prompt.device), None))
+                    # taken out for the call: calls from several threads have a pool each
+                    pool = self._pools.pop(str(prompt.device), None) or CapturePool(prompt.device)
+                    graph = StepGraph(bb, cache, step_in, pool)
                 except RuntimeError as err:    # what cannot be captured is issued directly, and raises there if it is wrong
                     warnings.warn(f"decode steps are issued one by one, their capture failed: {err}")
                     graphs = False
@@ -223,7 +250,7 @@ class LocalGenerator:
             if bool(finished.all()):
                 break
         if graph is not None:
-            self._captures[str(prompt.device)] = graph
+            self._pools[str(prompt.device)] = pool
         bb.train(was_training)
         return tokens
 

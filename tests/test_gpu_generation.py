@@ -106,3 +106,68 @@ def test_modes_see_every_decode_step():
         assert torch.equal(got, want)
         assert counts[2] - counts[1] == counts[1] - counts[0] > 8 * model.config.depth    # the same for each eight steps
     assert capturable(model, tokens)
+
+
+def test_other_threads_draw_random_numbers_while_steps_are_captured():
+    """A capture concerns the thread and the stream that it runs on: another thread's draws from the device's default
+    generator, allocations and launches go on meanwhile, on as many of torch's streams as there are."""
+    import threading
+
+    from kohakuwullm_b200.generation.engine import LocalGenerator
+    from kohakuwullm_b200.ops import native
+
+    model = _model()
+    tokens = torch.randint(1, 512, (1, 5), device="cuda")
+    gen = LocalGenerator(model, eos_id=511, stop_ids=(600,))
+    want = gen.generate(tokens, 7, temperature=0.0)
+    done, errors = threading.Event(), []
+
+    def draw():
+        streams = [torch.cuda.Stream() for _ in range(32)]
+        while not done.is_set():
+            for stream in streams:
+                try:
+                    with torch.cuda.stream(stream):
+                        assert float(torch.rand(1000, device="cuda").max()) <= 1.0
+                    draws.append(1)
+                except Exception as err:
+                    errors.append(err)
+                    return
+
+    draws = []
+    other = threading.Thread(target=draw)
+    other.start()
+    try:
+        got = [gen.generate(tokens, 7, temperature=0.0) for _ in range(60)]
+    finally:
+        done.set()
+        other.join()
+    torch.cuda.synchronize()
+    native.check_status()
+    assert not errors, errors[0]
+    assert len(draws) > 60 and all(torch.equal(g, want) for g in got)
+
+
+def test_captures_of_several_calls_take_over_their_memory():
+    """Calls after the first reserve no further memory, whatever the rows, and a generator that is dropped leaves none."""
+    import gc
+
+    from kohakuwullm_b200.generation.engine import LocalGenerator
+
+    model = _model()
+    prompts = [torch.randint(1, 512, (rows, 6), device="cuda") for rows in (4, 1, 3)]
+    LocalGenerator(model, eos_id=511, stop_ids=(600,)).generate(prompts[0], 9, temperature=0.0)    # what is made once
+    gc.collect()
+    torch.cuda.empty_cache()
+    start = torch.cuda.memory_allocated()
+    gen = LocalGenerator(model, eos_id=511, stop_ids=(600,))
+    first = [gen.generate(p, 9, temperature=0.0) for p in prompts]
+    reserved = torch.cuda.memory_reserved()
+    for _ in range(5):
+        assert all(torch.equal(gen.generate(p, 9, temperature=0.0), f) for p, f in zip(prompts, first))
+    assert torch.cuda.memory_reserved() == reserved
+    del gen, first
+    gc.collect()
+    assert torch.cuda.memory_allocated() == start
+    torch.cuda.empty_cache()
+    assert torch.cuda.memory_reserved() < reserved
