@@ -171,3 +171,29 @@ def test_captures_of_several_calls_take_over_their_memory():
     assert torch.cuda.memory_allocated() == start
     torch.cuda.empty_cache()
     assert torch.cuda.memory_reserved() < reserved
+
+
+def test_a_preview_leaves_no_memory_behind():
+    """The sampler of the in-training previews lives as long as the trainer and keeps no capture's memory from training."""
+    import gc
+
+    from kohakuwullm_b200.training.loop.sampling import PreviewSampler
+
+    class Tok:
+        bos_token_id = None
+        encode = staticmethod(lambda text: [ord(c) for c in text])
+        decode = staticmethod(lambda ids: " ".join(map(str, ids)))
+
+    model = _model()
+    prompt = torch.randint(1, 512, (2, 6), device="cuda")
+    sampler = PreviewSampler(eos_id=511)
+    for call in (lambda: sampler.generate(model, prompt, 9, temperature=0.0),
+                 lambda: sampler.texts(model, Tok, ["ab", "xyz"], 9, count=2, temperature=0.0)):
+        call()                                       # what is made once
+        gc.collect()
+        torch.cuda.empty_cache()
+        start = torch.cuda.memory_reserved()
+        call()
+        gc.collect()
+        torch.cuda.empty_cache()
+        assert torch.cuda.memory_reserved() == start and not sampler._pools
