@@ -123,13 +123,15 @@ def gemm(a_q, a_sf, b_q, b_sf, out=None, out_dtype=torch.bfloat16, accumulate=Fa
 
 
 # ------------------------------------------------------------------------------------ weights: tile width
-TILE_WIDTHS = (128, 144, 160, 176, 192, 208, 224, 240)
+# The widths that are chosen from: those of CTA pairs. A weight keeps its width for every product that it meets, and odd
+# multiples of 16 (which the kernel also takes) run on single CTAs whatever the rows.
+TILE_WIDTHS = (128, 160, 192, 224)
 
 
 def pick_tile_width(n_cols: int, m_rows: int = 4096, sms: int = 148) -> int:
     """Width of the output tiles of ``A (m_rows, K) x W (n_cols, K)^T`` that minimises rounds x cost per round.
 
-    Products of more than 128 rows run on pairs of SMs (256-row tiles, widths that are multiples of 32). A round of the
+    Products of more than 128 rows run on pairs of SMs (256-row tiles). A round of the
     pairs costs ``108 + BN`` units, fitted to B200 times of 14 products of 2048 to 8192 rows and K 1024 to 7168 (at K =
     1280: 3.1 us for 128 columns, 3.6 for 160, 3.9 for 192, 4.5 for 224), and a problem takes ``ceil(tiles / pairs)``
     rounds: 4096 x 1280 is three rounds of 128 columns or two of 160 (27.2 and 20.9 us at K = 3584), 4096 x 7168
@@ -142,8 +144,6 @@ def pick_tile_width(n_cols: int, m_rows: int = 4096, sms: int = 148) -> int:
     tiles_m = max((m_rows + 255) // 256 if pairs else (m_rows + 127) // 128, 1)
     best, best_bn = None, 128
     for bn in TILE_WIDTHS:
-        if pairs and bn % 32:
-            continue
         rounds = -(-(tiles_m * -(-n_cols // bn)) // (max(sms // 2, 1) if pairs else sms))
         cost = rounds * (108 + bn if pairs else 16 + bn / 8)
         if best is None or cost < best - 1e-9:
@@ -156,7 +156,7 @@ _TUNED: dict[tuple[int, int, int, int], int] = {}
 
 def tuned_tile_width(m_rows: int, n_cols: int, K: int, device) -> int:
     """Tile width for ``A (m_rows, K) x W (n_cols, K)^T``, MEASURED once per problem shape on this device: every
-    supported width runs the real kernel on synthetic operands (10 back-to-back launches between two events,
+    width of ``TILE_WIDTHS`` runs the real kernel on synthetic operands (10 back-to-back launches between two events,
     best of three) and the fastest wins; the result is cached. The analytic pick above ranks the widths by
     shared-memory traffic and wave count only and misses the fixed costs of a tile (pipeline fill, epilogue),
     which decide between near-equal candidates at short contraction lengths. Falls back to the analytic pick

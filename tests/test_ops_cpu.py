@@ -195,3 +195,13 @@ def test_blockwise_attention_fallback_matches_the_oracle_for_other_head_sizes():
             torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
     assert torch.equal(varlen_attention(q, k, v, info.cu_seqlens, window=40, sink_lse=sink),
                        varlen_attention_blockwise(q, k, v, info.cu_seqlens, 40, sink))      # the public entry point uses it
+
+
+def test_chosen_tile_widths_are_widths_of_cta_pairs():
+    """Wide weights quantised for few rows included: a width that only single CTAs run would stay with the weight."""
+    from kohakuwullm_b200.ops.mxfp8 import TILE_WIDTHS, pick_tile_width
+
+    assert all(bn % 32 == 0 for bn in TILE_WIDTHS)
+    for rows in (1, 64, 128, 129, 256, 512, 4096, 16384):
+        for cols in (128, 1280, 1296, 3584, 18944, 19072, 32768, 65536, 131072):
+            assert pick_tile_width(cols, rows) in TILE_WIDTHS
