@@ -53,7 +53,8 @@ class TimedLibrary:
     HOST_ONLY = ("kwu_last_error", "kwu_launch_count", "kwu_sumsq_blocks", "kwu_mxfp8_sf_bytes", "kwu_ce_tiles_n",
                  "kwu_flash_bwd_scratch_floats", "kwu_decode_scratch_floats", "kwu_rmsnorm_bwd_blocks",
                  "kwu_moe_max_rows", "kwu_ddp_blocks", "kwu_ep_flag_ints", "kwu_ep_table_ints", "kwu_sr_chunk_bytes",
-                 "kwu_gemm_debug_override")
+                 "kwu_stream_create", "kwu_stream_destroy", "kwu_capture_begin", "kwu_capture_end", "kwu_graph_launch",
+                 "kwu_graph_destroy")
 
     SHAPE_ARGS = {"kwu_gemm_mxfp8": (5, 6, 7), "kwu_gemm_bf16": (3, 4, 5)}
 

@@ -14,16 +14,16 @@
 // way (1316 us, 735 of them at the special-function rate, 1068 without them).
 //
 // SPLIT (cached prefill and other padded batches, which keep 32-bit probabilities): P leaves the softmax as three bf16
-// numbers, its rounding, the rounding of what that left out, and the rest: 8 + 8 + 8 bits hold an fp32 number exactly, and
-// O += P V runs once for each. The two lower parts overwrite score columns that the same thread has read, so their
+// numbers, its rounding, the rounding of what that left out, and the rest: 8 + 8 + 8 bits hold an fp32 number exactly,
+// and O += P V runs once for each. The two lower parts overwrite score columns that the same thread has read, so their
 // products are issued before the next tile's scores and the high one after them: the tensor pipe stays ahead of the
 // softmax, which is the bound. On sums that cancel, two parts (16 bits) were 10 to 20 times as far from 64 bits as the
-// explicit fp32 form; three are nearer than it inside one key tile, and 2e-7 of the sum of magnitudes off over 3001 keys
-// (2e-8 the explicit form), where the tensor pipe's own fp32 sums are what is left. On ordinary values both forms' errors
-// are the output's bf16 rounding and agree to 1e-6. The third part costs two prompts of 3001 tokens 0.55 of 10.0 ms. The rows of a padded batch are documents of one length, and
-// their tiles are loaded through maps with the row as a dimension of its own: what lies past a row's end reads as zero.
-// Read on into the next row, its values would meet probabilities of zero, and a NaN or infinity among them (0 x inf)
-// would enter the sums of this row.
+// explicit fp32 form; three are nearer than it inside one key tile, and 2e-7 of the sum of magnitudes off over 3001
+// keys (2e-8 the explicit form), where the tensor pipe's own fp32 sums are what is left. On ordinary values both forms'
+// errors are the output's bf16 rounding and agree to 1e-6. The third part costs two prompts of 3001 tokens 0.55 of 10.0
+// ms. The rows of a padded batch are documents of one length, and their tiles are loaded through maps with the row as a
+// dimension of its own: what lies past a row's end reads as zero. Read on into the next row, its values would meet
+// probabilities of zero, and a NaN or infinity among them (0 x inf) would enter the sums of this row.
 //
 // Documents never attend across their boundary: a tile's key range is clipped to its own document
 // and (with a window) to the last `window` positions. Sinks enter as sink_lse[h] = logsumexp of the

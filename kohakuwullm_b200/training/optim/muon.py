@@ -12,10 +12,10 @@ scaled into the iteration's convergence radius, two iterations are offered:
   ratio m / n is at least ``gram_aspect`` use the phases (2, 3); squarer ones run the five steps directly.
 
 Batching. All matrices of one shape (the q/k/v/o, MLP and stacked expert weights of every layer) are stacked
-and orthogonalised as ONE batch per product, up to ``ns_batch_elems`` elements at a time. On a B200 the batched
-products run on the tcgen05 grouped GEMM (every matrix of the batch is one "expert" of a grouped product: one
-launch per product for the whole batch, no transposes: ``X X^T`` and ``G G`` take both operands K-major, ``P X``
-takes X MN-major); elsewhere ``torch.bmm``.
+and orthogonalised as ONE batch per product, up to ``ns_batch_elems`` elements at a time. On a B200 a product of the
+whole batch is one launch of the tcgen05 GEMM over equal matrices (``kwu_gemm_bf16_batched``), without transposes:
+``X X^T`` and ``G G`` take both operands K-major, ``P X`` takes X MN-major, and the product that makes a phase's last
+``G`` writes ``a I + b G`` in its place. Elsewhere ``torch.bmm``.
 
 Write-back: ``p <- p (1 - lr wd) - lr scale U`` with ``scale`` = ``sqrt(max(1, rows / cols))`` (``spectral``) or
 ``rms_target sqrt(max(rows, cols))`` (``rms``); ``rounding="stochastic"`` rounds the bf16 result stochastically
