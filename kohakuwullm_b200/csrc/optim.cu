@@ -44,51 +44,43 @@ adamw_flat_kernel(float* __restrict__ master, float* __restrict__ m, float* __re
   const long long per_block = ((vecs + gridDim.x - 1) / gridDim.x + 31) & ~31LL;   // whole 512-byte lines of fp32
   const long long v_begin = static_cast<long long>(blockIdx.x) * per_block;
   const long long v_end = v_begin + per_block < vecs ? v_begin + per_block : vecs;
-  // Two vectors a thread and pass: their eight 16-byte loads are issued before the first is used. The segment of a vector
-  // lies at or after that of the thread's previous one, so it is found by walking on. 1.3 G parameters: 8.17 -> 7.80 ms.
+  // One vector a thread and pass; its segment lies at or after that of the thread's previous one, so it is found by walking
+  // on. Bound by HBM. us, a search per vector / this (bytes at the copy rate): 134 M elements in one segment 779 / 774
+  // (697), 546 M in 170 segments 3476 / 3116 (2834), 1.35 G in 500 segments 8706 / 7696 (7012). Streaming hints on the
+  // loads and stores cost 5 to 13 % (1.35 G: 8154, and 8820 with two vectors a pass), two vectors without them nothing
+  // but registers (7755).
   int s = v_begin + threadIdx.x < v_end ? find_segment(seg_start, nseg, (v_begin + threadIdx.x) << 2) : 0;
-  for (long long v0 = v_begin + threadIdx.x; v0 < v_end; v0 += 2LL * blockDim.x) {
-    float4 g4[2], p4[2], m4[2], v4[2];
+  for (long long vi = v_begin + threadIdx.x; vi < v_end; vi += blockDim.x) {
+    const long long i = vi << 2;
+    const float4 g4 = *reinterpret_cast<const float4*>(grad + i);
+    const float4 p4 = *reinterpret_cast<const float4*>(master + i);
+    const float4 m4 = *reinterpret_cast<const float4*>(m + i);
+    const float4 v4 = *reinterpret_cast<const float4*>(v + i);
+    // segments start on multiples of 4 elements, so one lookup serves the whole vector
+    while (s + 1 < nseg && seg_start[s + 1] <= i) ++s;
+    const float wd = seg_wd[s];
+    const float lr = hp.lr * seg_lr_mult[s];
+    float g[4] = {g4.x * gs, g4.y * gs, g4.z * gs, g4.w * gs};
+    float p[4] = {p4.x, p4.y, p4.z, p4.w};
+    float mm[4] = {m4.x, m4.y, m4.z, m4.w};
+    float vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const long long i = (v0 + u * static_cast<long long>(blockDim.x)) << 2;
-      if (i >> 2 < v_end) {
-        g4[u] = __ldcs(reinterpret_cast<const float4*>(grad + i));
-        p4[u] = __ldcs(reinterpret_cast<const float4*>(master + i));
-        m4[u] = __ldcs(reinterpret_cast<const float4*>(m + i));
-        v4[u] = __ldcs(reinterpret_cast<const float4*>(v + i));
-      }
+    for (int e = 0; e < 4; ++e) {
+      mm[e] = hp.beta1 * mm[e] + (1.f - hp.beta1) * g[e];
+      vv[e] = hp.beta2 * vv[e] + (1.f - hp.beta2) * g[e] * g[e];
+      const float denom = sqrtf(vv[e]) * hp.bc2_inv_sqrt + hp.eps;
+      p[e] = p[e] * (1.f - lr * wd) - lr * (mm[e] * hp.bc1_inv) / denom;
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const long long i = (v0 + u * static_cast<long long>(blockDim.x)) << 2;
-      if (i >> 2 >= v_end) break;
-      // segments start on multiples of 4 elements, so one lookup serves the whole vector
-      while (s + 1 < nseg && seg_start[s + 1] <= i) ++s;
-      const float wd = seg_wd[s];
-      const float lr = hp.lr * seg_lr_mult[s];
-      float g[4] = {g4[u].x * gs, g4[u].y * gs, g4[u].z * gs, g4[u].w * gs};
-      float p[4] = {p4[u].x, p4[u].y, p4[u].z, p4[u].w};
-      float mm[4] = {m4[u].x, m4[u].y, m4[u].z, m4[u].w};
-      float vv[4] = {v4[u].x, v4[u].y, v4[u].z, v4[u].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        mm[e] = hp.beta1 * mm[e] + (1.f - hp.beta1) * g[e];
-        vv[e] = hp.beta2 * vv[e] + (1.f - hp.beta2) * g[e] * g[e];
-        const float denom = sqrtf(vv[e]) * hp.bc2_inv_sqrt + hp.eps;
-        p[e] = p[e] * (1.f - lr * wd) - lr * (mm[e] * hp.bc1_inv) / denom;
-      }
-      __stcs(reinterpret_cast<float4*>(master + i), make_float4(p[0], p[1], p[2], p[3]));
-      __stcs(reinterpret_cast<float4*>(m + i), make_float4(mm[0], mm[1], mm[2], mm[3]));
-      __stcs(reinterpret_cast<float4*>(v + i), make_float4(vv[0], vv[1], vv[2], vv[3]));
-      if (param_lp) {
-        uint2 o;
-        o.x = pack_bf16(p[0], p[1]);
-        o.y = pack_bf16(p[2], p[3]);
-        *reinterpret_cast<uint2*>(param_lp + i) = o;
-      }
-      if (zero_grad) __stcs(reinterpret_cast<float4*>(grad + i), make_float4(0.f, 0.f, 0.f, 0.f));
+    *reinterpret_cast<float4*>(master + i) = make_float4(p[0], p[1], p[2], p[3]);
+    *reinterpret_cast<float4*>(m + i) = make_float4(mm[0], mm[1], mm[2], mm[3]);
+    *reinterpret_cast<float4*>(v + i) = make_float4(vv[0], vv[1], vv[2], vv[3]);
+    if (param_lp) {
+      uint2 o;
+      o.x = pack_bf16(p[0], p[1]);
+      o.y = pack_bf16(p[2], p[3]);
+      *reinterpret_cast<uint2*>(param_lp + i) = o;
     }
+    if (zero_grad) *reinterpret_cast<float4*>(grad + i) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
