@@ -110,7 +110,8 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // The same for rows of at most 32 * NV vectors: a lane keeps its NV vectors in registers, all loads issued before the
 // first use and every byte read once. The general form reads the row back for the second pass, which costs a lone row
 // (a decode step) a trip to the L2 and a full grid the issue slots
-// (us, read twice / kept: 16384 x 1536 38.6 / 33.6, 6002 x 1280 12.3 / 10.8, 3001 x 768 4.7 / 4.2, one row 3.7 / 3.3).
+// (us, read twice / kept: 16384 x 1536 38.6 / 33.6, 6002 x 1280 12.3 / 10.8, 3001 x 768 4.7 / 4.2, one row 3.7 / 3.3;
+// which row counts it serves: rmsnorm_fwd_impl).
 template <int NV, bool HAS_RES>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
@@ -1110,6 +1111,17 @@ static bool mx_shape_ok(const char* what, int rows, int cols) {
   return true;
 }
 
+// Rows that the register form has in work at once: eight warps in every block that fits on the GPU.
+template <int NV, bool HAS_RES>
+static int rmsnorm_fwd_rows_at_once() {
+  static const int rows = [] {
+    int blocks = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, rmsnorm_fwd_reg_kernel<NV, HAS_RES>, 256, 0);
+    return 148 * 8 * (blocks > 0 ? blocks : 1);
+  }();
+  return rows;
+}
+
 static int rmsnorm_fwd_impl(const void* x, const void* res, const float* w, void* y, void* h_out,
                             float* rstd, int rows, int cols, float eps, int one_plus, const MxOut mx, void* stream) {
   if (cols % 8) { set_last_error("rmsnorm: cols must be a multiple of 8"); return 7; }
@@ -1118,19 +1130,27 @@ static int rmsnorm_fwd_impl(const void* x, const void* res, const float* w, void
   const int grid = grid_for(rows, 8);
   // vectors of a lane: up to 8 stay in registers (rows of 2048). With the fp8 copy only up to 4: its conversions need the
   // registers (4096 x 1280 with the copy: 11.4 us in registers, 9.8 read twice; 8192 x 1024: 12.6 and 13.6)
+  // Its registers also leave fewer rows in work at once (2368 at 7 and 8 vectors, 3552 at 5 and 6), so a little more than one
+  // such wave pays for two: it runs up to one wave, and from two waves on up to 6 vectors. us in registers / read twice,
+  // inputs not in the L2: 4096 x 1536 14.3 / 12.3, 3001 x 2048 with residual 21.4 / 17.2, 16384 x 1792 with residual 57.3 /
+  // 51.2; 16384 x 1280 22.6 / 25.5, one row of 1280 8.2 / 10.2
   const int nv = (cols / 8 + 31) / 32;
   auto go = [&](auto kern, const void* r) {
     launch_k(kern, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)r, w, (__nv_bfloat16*)y,
              (__nv_bfloat16*)h_out, rstd, rows, cols, eps, one_plus, mx); kwu::count_launch();
   };
+  auto pays = [&](int at_once) { return rows <= at_once || (nv <= 6 && rows / 2 >= at_once); };
+  auto general = [&] { if (res) go(rmsnorm_fwd_kernel<true>, res); else go(rmsnorm_fwd_kernel<false>, nullptr); };
 #define KWU_RMS_FWD(n)                                                                                       \
   case n:                                                                                                    \
-    if (res) go(rmsnorm_fwd_reg_kernel<n, true>, res); else go(rmsnorm_fwd_reg_kernel<n, false>, nullptr);   \
+    if (!pays(res ? rmsnorm_fwd_rows_at_once<n, true>() : rmsnorm_fwd_rows_at_once<n, false>())) general();  \
+    else if (res) go(rmsnorm_fwd_reg_kernel<n, true>, res);                                                  \
+    else go(rmsnorm_fwd_reg_kernel<n, false>, nullptr);                                                      \
     break
   switch (mx.q && nv > 4 ? 0 : nv) {
     KWU_RMS_FWD(1); KWU_RMS_FWD(2); KWU_RMS_FWD(3); KWU_RMS_FWD(4); KWU_RMS_FWD(5); KWU_RMS_FWD(6); KWU_RMS_FWD(7); KWU_RMS_FWD(8);
     default:
-      if (res) go(rmsnorm_fwd_kernel<true>, res); else go(rmsnorm_fwd_kernel<false>, nullptr);
+      general();
   }
 #undef KWU_RMS_FWD
   return check_launch("rmsnorm_fwd");

@@ -138,3 +138,27 @@ def test_norm_weight_gradients_accumulate_into_main_grad():
     qknorm_rope(q.detach().requires_grad_(), qw2, ang.cos(), ang.sin()).backward(dq)
     assert qw2.grad is None
     torch.testing.assert_close(qw2.main_grad, qw.grad - 1.0, rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("cols", [256, 1024, 1280, 1536, 1792, 2048])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_forms_agree_around_a_wave(cols, residual):
+    """Row counts around one and two waves of the form that keeps its row in registers, where the rule turns to the form that
+    reads it twice and back: every row is, to the bit, what it is among few."""
+    from kohakuwullm_b200.ops import native
+    from kohakuwullm_b200.ops.elementwise import rmsnorm
+
+    torch.manual_seed(cols)
+    most = 148 * 8 * 12 + 1
+    x = torch.randn(most, cols, device="cuda").bfloat16()
+    res = torch.randn(most, cols, device="cuda").bfloat16() if residual else None
+    w = torch.rand(cols, device="cuda") + 0.5
+    run = lambda lo, hi: rmsnorm(x[lo:hi], w, residual=res[lo:hi]) if residual else (rmsnorm(x[lo:hi], w),)
+    with torch.no_grad():
+        few = [torch.cat(t) for t in zip(*(run(lo, min(lo + 1000, most)) for lo in range(0, most, 1000)))]
+        for waves in (1, 2, 3, 4, 5, 6, 8, 10, 12):
+            for rows in (148 * 8 * waves, 148 * 8 * waves + 1):
+                for got, want in zip(run(0, rows), few):
+                    assert torch.equal(got, want[:rows])
+    torch.cuda.synchronize()
+    native.check_status()
